@@ -91,9 +91,9 @@ def parse_args():
                     help="steps of the energy-drift run of both forms (0: skip)")
     ap.add_argument("--theta2", type=float, default=1.0,
                     help="second opening angle measured for both forms (0: skip)")
-    ap.add_argument("--walk-form", choices=["auto", "union", "lanes", "prefetch"],
+    ap.add_argument("--walk-form", choices=["auto", "team", "lanes", "prefetch"],
                     default="auto",
-                    help="the FP64 walk: chosen by timing (default), warp union, per lane, or "
+                    help="the FP64 walk: chosen by size and timing (default), team, per lane, or "
                          "per lane loading the next record early")
     ap.add_argument("--profile", choices=["fp64", "mixed", "adjoint", "batch", "config0"],
                     help="profiling entry: build the dwarf, run two force evaluations, exit")
@@ -507,7 +507,7 @@ def form_accuracy(pos, vel, mass, c_cfg, dev, seed=4096):
     return out
 
 
-WALK_FORM_NAMES = {0: "warp union", 1: "per lane", 2: "per lane, next record loaded early"}
+WALK_FORM_NAMES = {0: "team", 1: "per lane", 2: "per lane, next record loaded early"}
 
 
 def settle_walk_form(st, c):
@@ -716,13 +716,13 @@ def run_ours(args, dist):
         try:
             with open(PROFILE_TRAFFIC) as f:
                 prof = json.load(f)
-            rec = prof["fp64_walk_lanes" if info.walkForm >= 1 else "fp64_walk"]
+            rec = prof["fp64_walk_lanes" if info.walkForm >= 1 else "fp64_walk_team"]
             per_body = rec["dram_bytes"] / rec["n_bodies"]
             traffic = per_body * n
         except (OSError, KeyError, ValueError):
             traffic = None
     roofline = {"bound": "fp64",
-                "kernel": "k_walk_fp64_lanes" if info.walkForm >= 1 else "k_walk_fp64",
+                "kernel": "k_walk_fp64_lanes" if info.walkForm >= 1 else "k_walk_fp64_team",
                 "achieved": achieved,
                 "peak": peak64, "unit": "TFLOP/s", "frac": achieved / peak64,
                 "traffic": traffic,
@@ -892,7 +892,7 @@ def run_profile(args):
 def main():
     args = parse_args()
     global WALK_FORM
-    WALK_FORM = {"auto": -1, "union": 0, "lanes": 1, "prefetch": 2}[args.walk_form]
+    WALK_FORM = {"auto": -1, "team": 0, "lanes": 1, "prefetch": 2}[args.walk_form]
     if args.impl == "reference":
         # the reference arm is host-only: rank 0 runs it, other ranks exit without work
         os.environ.setdefault("WORLD_SIZE", "1")

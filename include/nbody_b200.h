@@ -352,18 +352,19 @@ NBodyCudaStatus nbSetStepCUDA(NBodyCudaState* st, int step);
  * arguments) and counted evaluations are always launched directly. */
 NBodyCudaStatus nbSetStepGraphCUDA(NBodyCudaState* st, int enable);
 
-/* The FP64 force walk's form: 0 walks the union of a warp's 32 tree paths node by node (the
- * lanes whose path holds the node doing it, one broadcast load per node); 1 walks every body's
- * path in its own lane (a lane idles only once its walk is over; per-lane loads); 2 is the
- * per-lane walk that loads the next node's record as soon as the opening test has chosen it,
- * overlapping that load with the current node's arithmetic (more registers: faster for small
- * systems, slower at a million bodies).  -1 (the default) cycles twice through the three
- * forms over a state's first six uncounted FP64 tree evaluations, times the second round (the
- * first launch of each kernel also loads it) and keeps the fastest.  Every form gives every
- * body exactly its CPU walk -- same nodes, same order, same sums: the accelerations are the
- * same bit for bit.  A batch walks the union unless its form is set (nbBatchSetWalkFormCUDA);
- * the force adjoint always walks the union (it reduces each node's adjoints over the warp).
- * nbGetWalkFormCUDA reports the form in use (-1 while undecided). */
+/* The FP64 force walk's form: 0 is the team walk for systems of up to 32,768 bodies (a warp walks
+ * for four bodies, eight lanes each evaluating the nodes of one body's path) and the per-lane walk
+ * above; 1 walks every body's path in its own lane (a lane idles only once its walk is over;
+ * per-lane loads); 2 is the per-lane walk that loads the next node's record as soon as the opening
+ * test has chosen it, overlapping that load with the current node's arithmetic (more registers:
+ * faster for some tens of thousands of bodies, slower at a million).  -1 (the default) takes the
+ * team walk up to 32,768 bodies; above, it cycles twice through forms 1 and 2 over a state's
+ * first four uncounted FP64 tree evaluations, times the second round (the first launch of each
+ * kernel also loads it) and keeps the faster.  Every form gives every body exactly its CPU walk --
+ * same nodes, same order, same sums: the accelerations are the same bit for bit.  A batch takes
+ * form 0 unless its form is set (nbBatchSetWalkFormCUDA); the force adjoint walks the union of a
+ * warp's paths (it reduces each node's adjoints over the warp).
+ * nbGetWalkFormCUDA reports the form in use (-1 before the first evaluation or while undecided). */
 NBodyCudaStatus nbSetWalkFormCUDA(NBodyCudaState* st, int form);
 NBodyCudaStatus nbGetWalkFormCUDA(NBodyCudaState* st, int* form);
 
@@ -495,8 +496,9 @@ NBodyCudaStatus nbBatchSetTuningCUDA(NBodyCudaBatch* batch, int groupMax, int li
 /* as nbSetMixedModeCUDA, for every dwarf of the batch */
 NBodyCudaStatus nbBatchSetMixedModeCUDA(NBodyCudaBatch* batch, int exactSet);
 /* The FP64 walk's form for every dwarf of the batch, as nbSetWalkFormCUDA but without the
- * automatic choice: 0 (the default) the warp union, 1 per lane, 2 per lane with the next
- * record loaded early (a warp may span two dwarfs; each lane walks only its own dwarf's tree). */
+ * automatic choice: 0 (the default) the team walk for batches of up to 32,768 bodies in all and
+ * per lane above, 1 per lane, 2 per lane with the next record loaded early (a warp may span two
+ * dwarfs; each body walks only its own dwarf's tree). */
 NBodyCudaStatus nbBatchSetWalkFormCUDA(NBodyCudaBatch* batch, int form);
 NBodyCudaStatus nbBatchGetTuningCUDA(NBodyCudaBatch* batch, int* groupMax, int* listCap,
                                      int* blocksPerSM);

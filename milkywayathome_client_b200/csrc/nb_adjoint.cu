@@ -5,7 +5,8 @@
 // mbar_j = sum_i abar_i . d a_i / d m_j for the accelerations of the last force evaluation,
 // keeping every opening decision of that evaluation (the tree is frozen).  Through the tree
 // the accelerations depend on the bodies via the cell moments, so the adjoint has two parts:
-//   1. k_walk_vjp: the same warp-union walk as k_walk_fp64 (nbody_grav.c:42-124); for every
+//   1. k_walk_vjp: a warp visits the union of its 32 bodies' walks (nbody_grav.c:42-124) node by
+//      node; for every
 //      interaction (body i, node q) it forms the tidal-tensor product
 //          dbar_r = m (abar s^-3/2 - 3 r (r.abar) s^-5/2)   (+ quadrupole terms)
 //      with r = x_q - x_i, s = |r|^2 + eps^2, subtracts it from body i and adds it, with the
@@ -392,7 +393,8 @@ void nb_launch_vjp(NbTreeBuffers& b, double* nodeBar, int capNodes, int maxDepth
     const int warps = (n + 31) / 32;
     cudaEventRecord(walkStart, s);
     // packed records from the (possibly restored) tree arrays
-    nb_launch_pack_walk(b.nodePM, b.nodeCrit, b.nodeLink, b.nodeQuad, b.walkRec, capNodes, b.sc, s);
+    nb_launch_pack_walk(b.nodePM, b.nodeCrit, b.nodeLink, b.nodeQuad, b.walkRec, b.walkKids, capNodes,
+                        b.sc, s);
     k_walk_vjp<<<(warps * 32 + 127) / 128, 128, 0, s>>>(b.walkRec, b.sort.idxA, b.px, b.py, b.pz,
                                                         abar, xbar, nodeBar, wp, pot, b.sc);
     cudaEventRecord(walkEnd, s);

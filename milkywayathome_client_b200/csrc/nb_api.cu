@@ -128,9 +128,9 @@ struct NbSlot {
     double lmc[6] = {0, 0, 0, 0, 0, 0};   // the LMC's position and velocity (LMC runs)
 };
 
-// The FP64 walk forms the automatic choice times (nbSetWalkFormCUDA): 0 the warp union,
+// The FP64 walk forms the automatic choice times above the team walk's line (nbSetWalkFormCUDA):
 // 1 the walk per lane, 2 the walk per lane that loads the next node's record early.
-static const int kWalkTuneForms[] = {0, 1, 2};
+static const int kWalkTuneForms[] = {1, 2};
 static const int kWalkTuneN = (int) (sizeof kWalkTuneForms / sizeof kWalkTuneForms[0]);
 
 struct NBodyCudaState {
@@ -183,9 +183,10 @@ struct NBodyCudaState {
     int useStepGraph = 1;
     int stepGraphForm = -1;
     NbScalars* scInit = nullptr;
-    // the FP64 walk's form (nbSetWalkFormCUDA): -1 chooses by timing -- the first 2C uncounted
-    // FP64 tree evaluations cycle twice through the C candidate forms, the second round (past
-    // each kernel's first launch, which also loads it) is timed, the fastest form is kept
+    // the FP64 walk's form (nbSetWalkFormCUDA): -1 takes the team walk where nb_walk_team(n) and
+    // chooses by timing above -- the first 2C uncounted FP64 tree evaluations cycle twice through
+    // the C candidate forms, the second round (past each kernel's first launch, which also loads
+    // it) is timed, the fastest form is kept
     int walkForm = -1;
     int walkFormChosen = -1;
     int walkTuneStep = 0;
@@ -218,6 +219,7 @@ static void nb_free_nodes(NBodyCudaState* st)
     cudaFree(b.nodeDepth); cudaFree(b.parent); cudaFree(b.nchild); cudaFree(b.arrive);
     cudaFree(b.nodeRange); b.nodeRange = nullptr;
     cudaFree(b.walkRec); b.walkRec = nullptr;
+    cudaFree(b.walkKids); b.walkKids = nullptr;
     cudaFree(st->mx.groups);
     cudaFree(st->mx.hi); cudaFree(st->mx.lo); cudaFree(st->mx.q32); cudaFree(st->mx.child8);
     b.nodePM = nullptr; b.nodeCrit = nullptr; b.nodeLink = nullptr; b.nodeQuad = nullptr;
@@ -244,6 +246,7 @@ static NBodyCudaStatus nb_alloc_nodes(NBodyCudaState* st, int cap)
     NB_CHECK(nb_alloc(&b.arrive, cap));
     NB_CHECK(nb_alloc(&b.nodeRange, cap));
     NB_CHECK(nb_alloc(&b.walkRec, 3 * (size_t) cap));
+    NB_CHECK(nb_alloc(&b.walkKids, 2 * (size_t) cap));
     NB_CHECK(nb_alloc(&st->mx.groups, cap));
     NB_CHECK(nb_alloc(&st->mx.hi, cap));
     NB_CHECK(nb_alloc(&st->mx.lo, cap));
@@ -476,6 +479,7 @@ static NBodyCudaStatus nb_force(const NBodyCudaCtx* ctx, NBodyCudaState* st, int
     if (fp64Tree) {
         if (st->walkForm >= 0) form = st->walkForm;
         else if (st->walkFormChosen >= 0) form = st->walkFormChosen;
+        else if (nb_walk_team(n)) form = st->walkFormChosen = 0;
         else { form = kWalkTuneForms[st->walkTuneStep % kWalkTuneN]; tuning = !st->counting; }
     }
     // The device work of the evaluation, enqueued without host synchronisation: the scalars
@@ -508,7 +512,7 @@ static NBodyCudaStatus nb_force(const NBodyCudaCtx* ctx, NBodyCudaState* st, int
             else
                 nb_launch_walk_fp64(b.nodePM, b.nodeCrit, b.nodeLink, b.nodeQuad, b.sort.idxA, b.px,
                                     b.py, b.pz, b.ax, b.ay, b.az, b.vx, b.vy, b.vz, wp, pot, b.sc,
-                                    st->counting != 0, s, b.walkRec, st->capNodes, nullptr,
+                                    st->counting != 0, s, b.walkRec, b.walkKids, st->capNodes, nullptr,
                                     form);
             rec(st->ev1);
         }
@@ -2103,7 +2107,7 @@ static int nb_batch_enqueue(NBodyCudaBatch* bt, const NBodyCudaCtx* ctx, int dri
     } else {
         nb_launch_walk_fp64(b.nodePM, b.nodeCrit, b.nodeLink, b.nodeQuad, b.sort.idxA, b.px, b.py,
                             b.pz, b.ax, b.ay, b.az, b.vx, b.vy, b.vz, wp, pot, b.sc, false, s,
-                            b.walkRec, st->capNodes, &f, st->walkForm > 0 ? st->walkForm : 0);
+                            b.walkRec, b.walkKids, st->capNodes, &f, st->walkForm > 0 ? st->walkForm : 0);
         launches += 1;
     }
     cudaEventRecord(st->ev1, s);

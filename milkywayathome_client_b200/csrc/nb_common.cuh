@@ -285,6 +285,7 @@ struct NbTreeBuffers {
     int *nodeDepth, *parent, *nchild, *arrive;
     int2* nodeRange;   // first and last sorted body of every node's subtree
     double4* walkRec;  // 3 per node: the FP64 walk's packed node records
+    int4* walkKids;    // 2 per node: a cell's children, up to 8 (-1: none)
     NbScalars* sc;
 };
 
@@ -306,18 +307,20 @@ size_t nb_mixed_stack_ints(int blocks);
 
 // The FP64 walks' packed node records (3 double4 per node) from the tree arrays.
 void nb_launch_pack_walk(const double4* nodePM, const double* nodeCrit, const int2* nodeLink,
-                         const double* nodeQuad, double4* rec, int capNodes, const NbScalars* sc,
-                         cudaStream_t s);
+                         const double* nodeQuad, double4* rec, int4* kids, int capNodes,
+                         const NbScalars* sc, cudaStream_t s);
 
 // The walks (forest != nullptr: one tree per dwarf, see NbForest).  form: the FP64 walk's
-// form, 0 the warp-union walk, 1 the walk per lane.
+// form, 0 the team walk where nb_walk_team(n) (else as 1), 1 the walk per lane, 2 per lane with
+// the next record loaded early.
+bool nb_walk_team(int n);
 void nb_launch_walk_fp64(const double4* nodePM, const double* nodeCrit, const int2* nodeLink,
                          const double* nodeQuad, const unsigned* order, const double* px,
                          const double* py, const double* pz, double* ax, double* ay, double* az,
                          double* vx, double* vy, double* vz, const NbWalkParams& wp,
                          const NbPot& pot, NbScalars* sc, bool count, cudaStream_t s,
-                         double4* walkRec, int capNodes, const NbForest* forest = nullptr,
-                         int form = 0);
+                         double4* walkRec, int4* walkKids, int capNodes,
+                         const NbForest* forest = nullptr, int form = 0);
 void nb_launch_walk_mixed(const NbTreeBuffers& b, const NbMixedBuffers& m, int capNodes,
                           const NbWalkParams& wp, const NbPot& pot, bool count, int numSMs,
                           cudaStream_t s, const NbForest* forest = nullptr);

@@ -2,31 +2,30 @@
 // potential.  Compiled with -fmad=false so every expression keeps the reference's rounding
 // (the reference CPU build uses SSE2 without FMA, milkyway/include/milkyway_math_double.h:128).
 //
-// Walk (nbGravity, nbody/src/nbody_grav.c:42-124).  One warp walks for 32 bodies that are
-// consecutive in octree-path order.  Every lane keeps its own position in the reference's
-// stackless walk: at node q it accepts (interacts, then jumps to Next(q)) if q is a body or
-// |dr|^2 >= rcrit2(q), otherwise it opens q (goes to More(q) = q + 1 in walk order).  Two
-// forms: the warp-union walk (k_walk_fp64) visits the smallest pending node of its lanes, each
-// node record read once per warp visit (uniform address); the per-lane walk
-// (k_walk_fp64_lanes) lets each lane take its own next node every iteration.  Either way each
-// lane sees exactly the nodes of its own CPU walk, in the CPU's order, and accumulates the same
-// terms in the same order.  A monopole interaction is 18 flops + sqrt + 2 divisions, a
-// quadrupole cell adds 38 flops + 2 divisions: the FP64 pipe (and, per lane, the L1 data pipe
-// that gathers the records) bounds the walk.
+// Walk (nbGravity, nbody/src/nbody_grav.c:42-124): the reference's stackless walk of every body.
+// At node q the body accepts (interacts, then jumps to Next(q)) if q is a body or |dr|^2 >=
+// rcrit2(q), otherwise it opens q (goes to More(q) = q + 1 in walk order).  Two kernels: the team
+// walk (k_walk_fp64_team) gives four bodies a warp and evaluates eight nodes at once for each, for
+// systems too small to fill the GPU with one lane a body; the per-lane walk (k_walk_fp64_lanes)
+// lets each lane walk its own body's path.  Either way each body gets exactly the nodes of its
+// own CPU walk, and sums the same terms in the CPU's order.  A monopole interaction is 18 flops
+// + sqrt + 2 divisions, a quadrupole cell adds 38 flops + 2 divisions.
 #include "nb_common.cuh"
 #include "nb_potential.cuh"
+#include "nb_rdiv.cuh"
 
 constexpr int WALK_THREADS = 128;
 
 // FOREST: the nodes hold one tree per dwarf (batched dwarfs); each lane walks its own
-// dwarf's tree, [rootNode, rootEnd), with that dwarf's softening and time step.  A warp whose
-// 32 bodies straddle two dwarfs visits the union of both walks, each lane its own.
+// dwarf's tree, [rootNode, rootEnd), with that dwarf's softening and time step.
 // The walk reads one packed record per node (k_pack_walk): 96 bytes, three double4 --
 // {CoM, mass}, {rcrit2, Next and body index as one 64-bit word, Qxx, Qxy},
-// {Qxz, Qyy, Qyz, Qzz} -- so a visit touches one record instead of four arrays.
+// {Qxz, Qyy, Qyz, Qzz} -- so a visit touches one record instead of four arrays -- and, for the
+// team walk, every cell's children (8 node numbers, -1 past the last).
 __global__ void k_pack_walk(const double4* __restrict__ nodePM, const double* __restrict__ nodeCrit,
                             const int2* __restrict__ nodeLink, const double* __restrict__ nodeQuad,
-                            double4* __restrict__ rec, const NbScalars* __restrict__ sc)
+                            double4* __restrict__ rec, int4* __restrict__ kids,
+                            const NbScalars* __restrict__ sc)
 {
     if (nb_failed(sc)) return;
     const int nNodes = sc->nNodes;
@@ -35,124 +34,289 @@ __global__ void k_pack_walk(const double4* __restrict__ nodePM, const double* __
         const long long word = (long long) (unsigned) l.x | ((long long) l.y << 32);
         const double* Q = nodeQuad + 6 * (size_t) k;
         const bool body = l.y >= 0;
-        rec[3 * (size_t) k] = nodePM[k];
-        rec[3 * (size_t) k + 1] = make_double4(nodeCrit[k], __longlong_as_double(word),
-                                               body ? 0.0 : Q[0], body ? 0.0 : Q[1]);
-        rec[3 * (size_t) k + 2] = body ? make_double4(0.0, 0.0, 0.0, 0.0)
-                                       : make_double4(Q[2], Q[3], Q[4], Q[5]);
+        double4* r = rec + 3 * (size_t) k;
+        r[0] = nodePM[k];
+        r[1] = make_double4(nodeCrit[k], __longlong_as_double(word), body ? 0.0 : Q[0],
+                            body ? 0.0 : Q[1]);
+        r[2] = body ? make_double4(0.0, 0.0, 0.0, 0.0) : make_double4(Q[2], Q[3], Q[4], Q[5]);
+        if (body) continue;
+        int ch[8] = {-1, -1, -1, -1, -1, -1, -1, -1};      // k + 1, then Next() up to Next(k)
+        int c = k + 1;
+#pragma unroll
+        for (int m = 0; m < 8; ++m)
+            if (c < l.x) { ch[m] = c; c = nodeLink[c].x; }
+        kids[2 * (size_t) k] = make_int4(ch[0], ch[1], ch[2], ch[3]);
+        kids[2 * (size_t) k + 1] = make_int4(ch[4], ch[5], ch[6], ch[7]);
     }
 }
 
+// The radial factors of one interaction at s = |dr|^2 + eps^2: mor3 = (m / sqrt(s)) / s, and for
+// a cell with quadrupole dr5inv = 1 / ((s s) sqrt(s)) and phiQ = 2.5 (dr5inv drQdr) / s, each
+// operation rounded as the reference's, with one reciprocal estimate for the root and all four
+// divisions (nb_rdiv.cuh).  2^-100 <= s < 2^100 and a mass and a numerator of phiQ between 2^-700
+// and 2^700 keep every intermediate and every residual normal; the operators take the rest, and
+// the divisors next to an all-ones significand.
+// ALWAYS: the quadrupole's factors are formed whether or not this lane's node is a cell (no branch).
+template <bool ALWAYS>
+__device__ __forceinline__ void nb_radial(double s, double m, bool need, bool cell, double drQdr,
+                                          double& mor3, double& dr5inv, double& phiQ)
+{
+    double y;
+    const double drab = nb_sqrt_recip(s, nb_rsqrt_estimate(s), y);
+    const double z = nb_recip_step(s, y * y);
+    mor3 = nb_quot(nb_quot(m, drab, y), s, z);
+    bool ok = nb_pos_exp_in<-100, 100>(s) && nb_exp_in<-700, 700>(m) && !nb_near_ones(s);
+    if (ALWAYS || cell) {
+        const double t = (s * s) * drab;
+        dr5inv = nb_recip_step(t, nb_recip_step(t, (z * z) * y));
+        const double a = 2.5 * (dr5inv * drQdr);
+        phiQ = nb_quot(a, s, z);
+        ok = ok && (!cell || (nb_exp_in<-700, 700>(a) && !nb_near_ones(t)));
+    }
+    if (need && !ok) {
+        const double root = sqrt(s);
+        mor3 = (m / root) / s;
+        if (cell) {
+            dr5inv = 1.0 / ((s * s) * root);
+            phiQ = 2.5 * (dr5inv * drQdr) / s;
+        }
+    }
+}
+
+// The team walk: a warp walks for TEAM_BODIES consecutive bodies, TEAM_LANES lanes each (lane =
+// TEAM_BODIES * p + b: lane p of body b's team).  The warp walks the union of its bodies' paths
+// depth first, a cell's children tested at once (lane p tests child p for body b, one ballot
+// gives every child's bodies), and lists the nodes that some body takes in walk order: a node
+// taken by a body is closed to it with all below (`cover`), a child that some body opens is
+// walked into before its later siblings.  Every TEAM_LANES listed nodes are evaluated at once, one
+// lane per (node, body); the terms go through shared memory to one lane per (body, component),
+// which adds them in list order while the next eight are evaluated -- every body sums its CPU
+// walk's terms in the CPU's order, and only the additions are serial.
+// What bounds it: latency (about 2.8 cycles a warp instruction wait on a dependent result) and,
+// at its upper end, issue slots: four bodies share ~200 instructions per eight nodes and ~150 per
+// opened cell, against ~190 a node for 32 bodies in the per-lane walk, which carries the
+// root-and-divisions chain of every node in its serial part on an eighth of the warps.  Five
+// resident blocks (96 registers): six to eight (80 to 64) were 3 to 20 % slower.
+// Walk times, per lane (the faster of its two forms, shared divisions) -> team, on the sampled
+// dwarf: 1,024 bodies (SW93, theta 1) 0.210 -> 0.106 ms, 5,000 (theta 1) 0.37 -> 0.155,
+// 20,000 (theta 1) 0.425 -> 0.333, (theta 0.5) 1.57 -> 1.07, 32,768 (theta 0.7) 0.861 -> 0.871,
+// 50,000 (theta 0.7) 0.996 -> 1.33.  Hence the line at TEAM_MAX_BODIES.
+constexpr int TEAM_BODIES = 4;
+constexpr int TEAM_MAX_BODIES = 32768;
+constexpr int TEAM_LANES = 32 / TEAM_BODIES;                // 8: a cell's children
+constexpr unsigned TEAM_ALL = (1u << TEAM_BODIES) - 1u;     // every body of the warp
+constexpr unsigned TEAM_FIRST = 0x11111111u;                // the lanes with b = 0
+constexpr int TEAM_RING = 16;         // at most 7 listed before a cell's up to 8
+struct NbTeam {
+    double term[3][3 * 32 + 4];         // component: three terms of every lane (padded)
+    int2 ring[TEAM_RING];               // listed: {node, cells complemented; bodies that take it}
+    // the cells with siblings below them still to list: {cell, the bodies of its eight children in
+    // four bits each, next child | cover << 8 | open children << 16 | children that are bodies << 24}
+    int4 frame[NB_GRID_LEVELS + 2];
+};
+
 template <bool COUNT, bool FOREST>
-__global__ void __launch_bounds__(WALK_THREADS)
-k_walk_fp64(const double4* __restrict__ rec,
+__global__ void __launch_bounds__(WALK_THREADS, 5)
+k_walk_fp64_team(const double4* __restrict__ rec, const int* __restrict__ kids,
             const unsigned int* __restrict__ order, const double* __restrict__ px,
             const double* __restrict__ py, const double* __restrict__ pz,
             double* __restrict__ ax, double* __restrict__ ay, double* __restrict__ az,
-            double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,
-            NbWalkParams wp, NbPot pot, NbScalars* __restrict__ sc, NbForest forest)
+            NbWalkParams wp, NbScalars* __restrict__ sc, NbForest forest)
 {
+    __shared__ NbTeam teams[WALK_THREADS / 32];
     if (nb_failed(sc)) return;
-    const int end = sc->nNodes;
+    NbTeam& T = teams[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    const int i = (int) ((blockIdx.x * (unsigned) blockDim.x + threadIdx.x) >> 5) * 32 + lane;
+    const int b = lane % TEAM_BODIES, p = lane / TEAM_BODIES;
+    const int i = (int) ((blockIdx.x * (unsigned) blockDim.x + threadIdx.x) >> 5) * TEAM_BODIES + b;
+    if (i - b >= wp.n) return;                      // the whole warp
     const bool valid = i < wp.n;
-    const unsigned j = valid ? order[i] : 0u;
+    const unsigned j = valid ? order[i] : 0xffffffffu;
     const double x0 = valid ? px[j] : 0.0, y0 = valid ? py[j] : 0.0, z0 = valid ? pz[j] : 0.0;
     double eps2 = wp.eps2;
     const bool useQuad = wp.useQuad != 0;
-    int start = 0, myEnd = end;
-    NbDwarfDev* dw = nullptr;
+    int root = 0;
     if (FOREST && valid) {
-        dw = &forest.dwarfs[forest.bodyDwarf[i]];
-        eps2 = dw->eps2;
-        wp.dtHalf = 0.5 * dw->dt;
-        start = dw->rootNode;
-        myEnd = dw->rootEnd;
+        const NbDwarfDev& dw = forest.dwarfs[forest.bodyDwarf[i]];
+        eps2 = dw.eps2;
+        root = dw.rootNode;
     }
-    int ptr = valid ? start : end;
-    double accx = 0.0, accy = 0.0, accz = 0.0;
+    double acc = 0.0;                   // lanes 0..11: component p of body b
     bool metSelf = false;
     unsigned long long cVisit = 0, cBB = 0, cBC = 0, cSteps = 0;
-    for (;;) {
-        if (FOREST && ptr >= myEnd) ptr = end;          // this lane's tree is done
-        const int q = __reduce_min_sync(NB_FULL_MASK, ptr);
-        if (q >= end) break;
-        if (COUNT) ++cSteps;
-        if (ptr != q) continue;
-        const double4 nd = nb_ld32(rec + 3 * (size_t) q);
-        const double4 r1 = nb_ld32(rec + 3 * (size_t) q + 1);
-        const long long word = __double_as_longlong(r1.y);
-        const int2 link = make_int2((int) (unsigned) (word & 0xffffffffll), (int) (word >> 32));
+
+    // the current cell's children, child p in lanes 4 p ..: node, the bodies that take it
+    int kid = -1, cellNode = -1;
+    unsigned use = 0;
+    unsigned todo = __ballot_sync(NB_FULL_MASK, valid) & TEAM_ALL;   // bodies whose tree is to come
+    unsigned open = 0, leaf = 0;        // bit 4 p: some body opens child p; child p is a body
+    unsigned cover = 0;                 // bodies that took an ancestor of these children
+    int pos = TEAM_LANES;               // the next child to list
+    int level = 0, head = 0, tail = 0;
+
+    // the opening test (nbody/src/nbody_grav.c:55-62) of the children in `kid`
+    auto test = [&]() {
+        const double4* r = rec + 3 * (size_t) max(kid, 0);
+        const double4 nd = nb_ld32(r);
+        const double2 r1 = __ldg(reinterpret_cast<const double2*>(r + 1));
+        const int bodyIndex = __double2hiint(r1.y);
         const double dx = nd.x - x0, dy = nd.y - y0, dz = nd.z - z0;
-        double drSq = dz * dz + (dy * dy + dx * dx);
-        const bool isBody = link.y >= 0;
-        if (COUNT) ++cVisit;
-        if (isBody || drSq >= r1.x) {
-            ptr = link.x;
-            if (isBody && (unsigned) link.y == j) { metSelf = true; continue; }
-            if (COUNT) { if (isBody) ++cBB; else ++cBC; }
-            drSq = drSq + eps2;
-            const double drab = sqrt(drSq);
-            const double phii = nd.w / drab;
-            const double mor3 = phii / drSq;
-            accx = accx + mor3 * dx;
-            accy = accy + mor3 * dy;
-            accz = accz + mor3 * dz;
-            if (useQuad && !isBody) {
-                const double4 r2 = nb_ld32(rec + 3 * (size_t) q + 2);
-                const double qxx = r1.z, qxy = r1.w, qxz = r2.x, qyy = r2.y, qyz = r2.z, qzz = r2.w;
-                const double qdx = qxx * dx + qxy * dy + qxz * dz;
-                const double qdy = qxy * dx + qyy * dy + qyz * dz;
-                const double qdz = qxz * dx + qyz * dy + qzz * dz;
-                const double drQdr = qdx * dx + qdy * dy + qdz * dz;
-                const double dr5inv = 1.0 / ((drSq * drSq) * drab);
-                const double phiQ = 2.5 * (dr5inv * drQdr) / drSq;
-                accx = accx + phiQ * dx;
-                accy = accy + phiQ * dy;
-                accz = accz + phiQ * dz;
-                accx = accx - dr5inv * qdx;
-                accy = accy - dr5inv * qdy;
-                accz = accz - dr5inv * qdz;
+        const double drSq = dz * dz + (dy * dy + dx * dx);
+        const bool mine = kid >= 0 && !((cover >> b) & 1u);     // this body still walks here
+        const bool body = kid >= 0 && bodyIndex >= 0;
+        const bool self = mine && body && (unsigned) bodyIndex == j;
+        const bool take = mine && (body ? !self : drSq >= r1.x);
+        metSelf |= self;
+        use = (__ballot_sync(NB_FULL_MASK, take) >> (TEAM_BODIES * p)) & TEAM_ALL;
+        leaf = __ballot_sync(NB_FULL_MASK, body) & TEAM_FIRST;
+        open = __ballot_sync(NB_FULL_MASK, kid >= 0 && !body && (cover | use) != TEAM_ALL) & TEAM_FIRST;
+        pos = 0;
+        if (COUNT) {
+            cVisit += __popc(__ballot_sync(NB_FULL_MASK, mine));
+            cBB += __popc(__ballot_sync(NB_FULL_MASK, take && body));
+            cBC += __popc(__ballot_sync(NB_FULL_MASK, take && !body));
+            ++cSteps;
+        }
+    };
+    // adds the last batch's terms in list order (every lane, for the arithmetic to overlap the
+    // next batch's; a zero term of either sign leaves the sum, which never is -0, as it is)
+    const double* const sums = T.term[min(p, 2)] + b;
+    auto add_terms = [&]() {
+#pragma unroll
+        for (int e = 0; e < TEAM_LANES; ++e) {
+            acc = acc + sums[TEAM_BODIES * e];
+            acc = acc + sums[32 + TEAM_BODIES * e];
+            acc = acc - sums[64 + TEAM_BODIES * e];
+        }
+    };
+    // the terms of up to TEAM_LANES listed nodes (nbody/src/nbody_grav.c:64-100)
+    auto evaluate = [&]() {
+        if (COUNT) ++cSteps;
+        const int2 entry = T.ring[(tail + p) % TEAM_RING];
+        const bool take = tail + p < head && (((unsigned) entry.y >> b) & 1u);
+        const int node = take ? (entry.x < 0 ? ~entry.x : entry.x) : 0;
+        const bool cell = entry.x < 0 && useQuad && take;
+        const double4* r = rec + 3 * (size_t) node;
+        const double4 nd = nb_ld32(r);
+        const double2 r1 = __ldg(reinterpret_cast<const double2*>(r + 1) + 1);
+        const double4 r2 = nb_ld32(r + 2);
+        add_terms();
+        const double dx = nd.x - x0, dy = nd.y - y0, dz = nd.z - z0;
+        const double s = (dz * dz + (dy * dy + dx * dx)) + eps2;
+        const double qxx = r1.x, qxy = r1.y, qxz = r2.x, qyy = r2.y, qyz = r2.z, qzz = r2.w;
+        const double qdx = qxx * dx + qxy * dy + qxz * dz;
+        const double qdy = qxy * dx + qyy * dy + qyz * dz;
+        const double qdz = qxz * dx + qyz * dy + qzz * dz;
+        const double drQdr = qdx * dx + qdy * dy + qdz * dz;
+        double mor3, dr5inv, phiQ;
+        nb_radial<true>(s, nd.w, take, cell, drQdr, mor3, dr5inv, phiQ);
+        __syncwarp();
+        T.term[0][lane] = take ? mor3 * dx : 0.0;
+        T.term[1][lane] = take ? mor3 * dy : 0.0;
+        T.term[2][lane] = take ? mor3 * dz : 0.0;
+        T.term[0][32 + lane] = cell ? phiQ * dx : 0.0;
+        T.term[1][32 + lane] = cell ? phiQ * dy : 0.0;
+        T.term[2][32 + lane] = cell ? phiQ * dz : 0.0;
+        T.term[0][64 + lane] = cell ? dr5inv * qdx : 0.0;
+        T.term[1][64 + lane] = cell ? dr5inv * qdy : 0.0;
+        T.term[2][64 + lane] = cell ? dr5inv * qdz : 0.0;
+        __syncwarp();
+        tail += TEAM_LANES;
+    };
+
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        T.term[0][32 * k + lane] = T.term[1][32 * k + lane] = T.term[2][32 * k + lane] = 0.0;
+    __syncwarp();
+    for (;;) {
+        if (pos >= TEAM_LANES) {                    // this cell's children are done
+            if (level > 0) {
+                --level;
+                __syncwarp();
+                const int4 f = T.frame[level];
+                cellNode = f.x;
+                kid = __ldg(kids + 8 * (size_t) cellNode + p);
+                use = ((unsigned) f.y >> (4 * p)) & TEAM_ALL;
+                pos = f.z & 255;
+                cover = ((unsigned) f.z >> 8) & 255u;
+                open = (unsigned) f.w & TEAM_FIRST;
+                leaf = ((unsigned) f.w >> 1) & TEAM_FIRST;
+            } else if (todo) {                      // the next root (one tree per dwarf)
+                const int r = __shfl_sync(NB_FULL_MASK, root, __ffs(todo) - 1);
+                const unsigned group = __ballot_sync(NB_FULL_MASK, valid && root == r) & TEAM_ALL;
+                todo &= ~group;
+                cover = TEAM_ALL & ~group;
+                kid = p == 0 ? r : -1;
+                test();
+            } else {
+                break;
             }
-        } else {
-            ptr = q + 1;
+        }
+        // list the children up to the next one that some body opens
+        const unsigned om = open & (~0u << (TEAM_BODIES * pos));
+        const int stop = om ? (__ffs(om) - 1) / TEAM_BODIES : TEAM_LANES - 1;
+        const unsigned taken = __ballot_sync(NB_FULL_MASK, b == 0 && use != 0u);
+        const unsigned adds = taken & (~0u << (TEAM_BODIES * pos)) &
+                              (~0u >> (TEAM_BODIES * (TEAM_LANES - 1 - stop)));
+        if ((adds >> lane) & 1u)
+            T.ring[(head + __popc(adds & ((1u << lane) - 1u))) % TEAM_RING] =
+                make_int2((leaf >> lane) & 1u ? kid : ~kid, (int) use);
+        head += __popc(adds);
+        pos = stop + 1;
+        if (om) {                                   // walk into it
+            const int c = __shfl_sync(NB_FULL_MASK, kid, TEAM_BODIES * stop);
+            const unsigned u = __shfl_sync(NB_FULL_MASK, use, TEAM_BODIES * stop);
+            const int next = __ldg(kids + 8 * (size_t) c + p);
+            if (pos < TEAM_LANES && ((taken | open) >> (TEAM_BODIES * pos)) != 0u) {
+                const unsigned uses = __reduce_or_sync(NB_FULL_MASK, use << (4 * p));
+                if (lane == 0)
+                    T.frame[level] = make_int4(cellNode, (int) uses, pos | (int) (cover << 8),
+                                               (int) (open | leaf << 1));
+                ++level;
+            }
+            cover |= u;
+            cellNode = c;
+            kid = next;
+            test();
+        }
+        if (head - tail >= TEAM_LANES) {
+            __syncwarp();
+            evaluate();
         }
     }
-    if (COUNT) {
-        for (int o = 16; o > 0; o >>= 1) {
-            cVisit += __shfl_xor_sync(NB_FULL_MASK, cVisit, o);
-            cBB += __shfl_xor_sync(NB_FULL_MASK, cBB, o);
-            cBC += __shfl_xor_sync(NB_FULL_MASK, cBC, o);
-        }
-        if (lane == 0) {
-            atomicAdd(&sc->nWarpSteps, cSteps);
-            atomicAdd(&sc->nVisit, cVisit);
-            atomicAdd(&sc->nBodyBody, cBB);
-            atomicAdd(&sc->nBodyCell, cBC);
-        }
+    __syncwarp();
+    if (tail < head) evaluate();
+    add_terms();
+    if (COUNT && lane == 0) {           // every lane counted the warp's numbers alike
+        atomicAdd(&sc->nWarpSteps, cSteps);
+        atomicAdd(&sc->nVisit, cVisit);
+        atomicAdd(&sc->nBodyBody, cBB);
+        atomicAdd(&sc->nBodyCell, cBC);
     }
+    // the team's lanes met the children between them
+    metSelf = (__ballot_sync(NB_FULL_MASK, metSelf) & (TEAM_FIRST << b)) != 0u;
     if (!valid) return;
     // a body that never meets itself is tree incest (nbody/src/nbody_grav.c:111-118)
-    if (!metSelf) {
+    if (p == 0 && !metSelf) {
         atomicOr(&sc->incest, 1);
-        if (FOREST) atomicOr(&dw->status, NBODY_TREE_INCEST_NONFATAL);
+        if (FOREST)
+            atomicOr(&forest.dwarfs[forest.bodyDwarf[i]].status, NBODY_TREE_INCEST_NONFATAL);
     }
     // self-gravity only; k_body_epilogue adds the external potential and kicks (kept out of
     // this kernel so that its registers serve the walk)
-    ax[j] = accx; ay[j] = accy; az[j] = accz;
+    if (p < 3) (p == 0 ? ax : p == 1 ? ay : az)[j] = acc;
 }
 
-// The same walk with every lane on its own path (no warp union): each iteration every lane
+// The walk with every lane on its own path: each iteration every lane
 // that has not finished takes the next node of its own walk (a per-lane gather of the node
-// record, one 32-byte load per sector, instead of one broadcast), so a lane is idle only when
-// its walk is over.  Each lane still meets exactly its CPU walk's nodes in the CPU's order and
-// sums the same terms in the same order.  Bodies consecutive in path order have walks of
-// similar length, so the warp runs about as many iterations as its longest walk, while the
-// union walk runs one iteration per node any of its lanes visits: on the 131k-body dwarf at
-// theta 0.5, 0.96 of the lane slots do work against 0.70 in the union walk (a CPU count over
-// the oracle's tree).  Walks in groups of 2 to 16 lanes (the union of each group's paths) were
-// measured between the two and slower than both.
+// record, one 32-byte load per sector), so a lane is idle only when its walk is over.  Each lane
+// meets exactly its CPU walk's nodes in the CPU's order and sums the same terms in the same
+// order.  Bodies consecutive in path order have walks of similar length, so the warp runs about
+// as many iterations as its longest walk (0.96 of the lane slots do work on the 131k-body dwarf
+// at theta 0.5).  Bound by the L1 data pipe (87 % busy: a 32-byte load is at least eight
+// wavefronts a warp, more with distinct records) and the FP64 pipe (63 %).  Sharing one
+// reciprocal among the root and the divisions (nb_radial) took the 1,048,576-body dwarf from 28.9
+// to 28.1 ms at theta 0.5 and from 7.05 to 6.54 ms at theta 1.
 template <bool COUNT, bool FOREST, bool PREFETCH>
 __global__ void __launch_bounds__(WALK_THREADS)
 k_walk_fp64_lanes(const double4* __restrict__ rec,
@@ -221,21 +385,21 @@ k_walk_fp64_lanes(const double4* __restrict__ rec,
         else if (accept) {
             if (COUNT) { if (isBody) ++cBB; else ++cBC; }
             drSq = drSq + eps2;
-            const double drab = sqrt(drSq);
-            const double phii = nd.w / drab;
-            const double mor3 = phii / drSq;
+            const bool quad = useQuad && !isBody;
+            double qdx, qdy, qdz, drQdr = 0.0, mor3, dr5inv, phiQ;
+            if (quad) {
+                const double4 r2 = nb_ld32(rec + 3 * (size_t) q + 2);
+                const double qxx = r1.z, qxy = r1.w, qxz = r2.x, qyy = r2.y, qyz = r2.z, qzz = r2.w;
+                qdx = qxx * dx + qxy * dy + qxz * dz;
+                qdy = qxy * dx + qyy * dy + qyz * dz;
+                qdz = qxz * dx + qyz * dy + qzz * dz;
+                drQdr = qdx * dx + qdy * dy + qdz * dz;
+            }
+            nb_radial<false>(drSq, nd.w, true, quad, drQdr, mor3, dr5inv, phiQ);
             accx = accx + mor3 * dx;
             accy = accy + mor3 * dy;
             accz = accz + mor3 * dz;
-            if (useQuad && !isBody) {
-                const double4 r2 = nb_ld32(rec + 3 * (size_t) q + 2);
-                const double qxx = r1.z, qxy = r1.w, qxz = r2.x, qyy = r2.y, qyz = r2.z, qzz = r2.w;
-                const double qdx = qxx * dx + qxy * dy + qxz * dz;
-                const double qdy = qxy * dx + qyy * dy + qyz * dz;
-                const double qdz = qxz * dx + qyz * dy + qzz * dz;
-                const double drQdr = qdx * dx + qdy * dy + qdz * dz;
-                const double dr5inv = 1.0 / ((drSq * drSq) * drab);
-                const double phiQ = 2.5 * (dr5inv * drQdr) / drSq;
+            if (quad) {
                 accx = accx + phiQ * dx;
                 accy = accy + phiQ * dy;
                 accz = accz + phiQ * dz;
@@ -489,53 +653,64 @@ void nb_launch_body_epilogue(const double* px, const double* py, const double* p
                              int numSMs, cudaStream_t s, const NbForest* forest);
 
 void nb_launch_pack_walk(const double4* nodePM, const double* nodeCrit, const int2* nodeLink,
-                         const double* nodeQuad, double4* rec, int capNodes, const NbScalars* sc,
-                         cudaStream_t s)
+                         const double* nodeQuad, double4* rec, int4* kids, int capNodes,
+                         const NbScalars* sc, cudaStream_t s)
 {
     k_pack_walk<<<min((capNodes + 255) / 256, 4096), 256, 0, s>>>(nodePM, nodeCrit, nodeLink,
-                                                                  nodeQuad, rec, sc);
+                                                                  nodeQuad, rec, kids, sc);
     nb_count_launch();
 }
+
+// The team walk below its line (form 0 is the per-lane walk above it).
+bool nb_walk_team(int n) { return n <= TEAM_MAX_BODIES; }
 
 void nb_launch_walk_fp64(const double4* nodePM, const double* nodeCrit, const int2* nodeLink,
                          const double* nodeQuad, const unsigned* order, const double* px,
                          const double* py, const double* pz, double* ax, double* ay, double* az,
                          double* vx, double* vy, double* vz, const NbWalkParams& wp,
                          const NbPot& pot, NbScalars* sc, bool count, cudaStream_t s,
-                         double4* walkRec, int capNodes, const NbForest* forest, int form)
+                         double4* walkRec, int4* walkKids, int capNodes, const NbForest* forest,
+                         int form)
 {
     const int warps = (wp.n + 31) / 32;
     const int blocks = (warps * 32 + WALK_THREADS - 1) / WALK_THREADS;
     if (blocks <= 0) return;
-    nb_launch_pack_walk(nodePM, nodeCrit, nodeLink, nodeQuad, walkRec, capNodes, sc, s);
+    nb_launch_pack_walk(nodePM, nodeCrit, nodeLink, nodeQuad, walkRec, walkKids, capNodes, sc, s);
     const NbForest f = forest ? *forest : NbForest{nullptr, nullptr, 0};
-#define NB_WALK_ARGS walkRec, order, px, py, pz, ax, ay, az, vx, vy, vz, wp, pot, sc, f
+    const bool team = form == 0 && nb_walk_team(wp.n);
+    const int perTeamBlock = TEAM_BODIES * WALK_THREADS / 32;
+    const int teamBlocks = (wp.n + perTeamBlock - 1) / perTeamBlock;
 #define NB_LANES_ARGS walkRec, order, px, py, pz, ax, ay, az, wp, sc, f
+#define NB_TEAM_ARGS walkRec, (const int*) walkKids, order, px, py, pz, ax, ay, az, wp, sc, f
+#define NB_TEAM(FOREST)                                                                       \
+    do {                                                                                      \
+        if (count) k_walk_fp64_team<true, FOREST><<<teamBlocks, WALK_THREADS, 0, s>>>(NB_TEAM_ARGS); \
+        else k_walk_fp64_team<false, FOREST><<<teamBlocks, WALK_THREADS, 0, s>>>(NB_TEAM_ARGS);    \
+    } while (0)
     if (forest) {
         if (form == 2) {
             if (count) k_walk_fp64_lanes<true, true, true><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
             else k_walk_fp64_lanes<false, true, true><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
-        } else if (form == 1) {
+        } else if (form == 1 || !team) {
             if (count) k_walk_fp64_lanes<true, true, false><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
             else k_walk_fp64_lanes<false, true, false><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
         } else {
-            if (count) k_walk_fp64<true, true><<<blocks, WALK_THREADS, 0, s>>>(NB_WALK_ARGS);
-            else k_walk_fp64<false, true><<<blocks, WALK_THREADS, 0, s>>>(NB_WALK_ARGS);
+            NB_TEAM(true);
         }
     } else {
         if (form == 2) {
             if (count) k_walk_fp64_lanes<true, false, true><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
             else k_walk_fp64_lanes<false, false, true><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
-        } else if (form == 1) {
+        } else if (form == 1 || !team) {
             if (count) k_walk_fp64_lanes<true, false, false><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
             else k_walk_fp64_lanes<false, false, false><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
         } else {
-            if (count) k_walk_fp64<true, false><<<blocks, WALK_THREADS, 0, s>>>(NB_WALK_ARGS);
-            else k_walk_fp64<false, false><<<blocks, WALK_THREADS, 0, s>>>(NB_WALK_ARGS);
+            NB_TEAM(false);
         }
     }
-#undef NB_WALK_ARGS
+#undef NB_TEAM
 #undef NB_LANES_ARGS
+#undef NB_TEAM_ARGS
     nb_count_launch();
     nb_launch_body_epilogue(px, py, pz, ax, ay, az, vx, vy, vz, wp, pot, sc, 0, s, forest);
 }

@@ -1,0 +1,74 @@
+"""The team walk (form 0 of the FP64 walk) at the sizes where it can go wrong, on a GPU: fewer
+bodies than a team, remainders, both sides of its line, and operands its shared reciprocals
+leave to the operators.  The accelerations equal the oracle's (small sizes) and the per-lane
+walk's bit for bit."""
+import numpy as np
+import pytest
+
+from conftest import bits_equal, make_ctx
+
+pytestmark = pytest.mark.gpu
+
+
+def _acc(ctx, pos, vel, mass, form):
+    from milkywayathome_client_b200 import NBodyState
+    with NBodyState.create(ctx, pos, vel, mass, gravmap=False) as st:
+        st.set_walk_form(form)
+        rc = st.gravMap(ctx)
+        return rc, st.accels()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 7, 8, 9, 15, 17, 31, 33, 1000, 1025])
+@pytest.mark.parametrize("cfg", [dict(theta=0.5), dict(theta=1.0, criterion="SW93"),
+                                 dict(theta=0.8, useQuad=False), dict(theta=0.0)],
+                         ids=["t0.5", "sw93", "noquad", "t0"])
+def test_small_sizes_equal_the_oracle(n, cfg):
+    from milkywayathome_client_b200 import models
+    from oracle import bindings as ob
+    pos, vel, mass, _ = models.plummer_plummer_dwarf(n, seed=40 + n)
+    ctx = make_ctx(max(n, 2), **cfg)
+    rc, want, _, _ = ob.grav_map(ctx.struct, pos, mass, ctx.treeRSize)
+    got_rc, got = _acc(ctx, pos, vel, mass, 0)
+    assert got_rc == rc and bits_equal(got, want)
+
+
+@pytest.mark.parametrize("n", [32767, 32768, 32769])
+def test_both_sides_of_the_line_equal_the_per_lane_walk(n):
+    from milkywayathome_client_b200 import models
+    pos, vel, mass, _ = models.plummer_plummer_dwarf(n, seed=5)
+    ctx = make_ctx(n, theta=0.9)
+    a, b = (_acc(ctx, pos, vel, mass, f) for f in (0, 1))
+    assert a[0] == b[0] == 0 and bits_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("case", ["no softening", "tiny masses", "huge masses", "tiny sizes",
+                                  "massless bodies", "near ones"])
+def test_operands_outside_the_shared_ranges(case):
+    from milkywayathome_client_b200 import _lib, models
+    from oracle import bindings as ob
+    n = 700
+    pos, vel, mass, _ = models.plummer_plummer_dwarf(n, seed=8)
+    over = dict(theta=0.7, potential=None, allowIncest=True)
+    if case == "no softening":
+        over["eps2"] = 0.0
+    elif case == "tiny masses":
+        mass = mass * 2.0 ** -715
+    elif case == "huge masses":
+        mass = mass * 2.0 ** 705
+    elif case == "tiny sizes":
+        over["eps2"] = 2.0 ** -120
+    elif case == "massless bodies":
+        mass = mass.copy()
+        mass[::9] = 0.0
+    else:
+        # softened distances next to powers of two: s = 4 - 2^-k and neighbours
+        pos = np.round((pos - pos.mean(0)) * 2.0) / 2.0
+        pos += np.arange(n)[:, None] * 2.0 ** -40
+        over["eps2"] = 4.0 - 2.0 ** -50
+    ctx = make_ctx(n, **over)
+    rc, want, _, _ = ob.grav_map(ctx.struct, pos, mass, ctx.treeRSize)
+    for form in (0, 1, 2):
+        got_rc, got = _acc(ctx, pos, vel, mass, form)
+        assert got_rc == rc, form
+        if not _lib.status_is_fatal(rc):
+            assert np.array_equal(got, want, equal_nan=True), form

@@ -1,0 +1,130 @@
+"""The shared-reciprocal root and divisions of the FP64 walk (csrc/nb_rdiv.cuh), no GPU.
+
+The header uses only fma, * and integer operations after the reciprocal estimate, so a host
+build of it computes what the device computes from an estimate of the same quality (the host's
+keeps 20 bits of 1/sqrt(s), as the device's instruction does).  Every result must equal the IEEE
+operator's, bit for bit: on random operands over the exponent ranges the walk admits, and on
+roots and quotients constructed to lie next to a rounding boundary.
+"""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                    "milkywayathome_client_b200", "csrc")
+SRC = r'''
+#include "nb_rdiv.cuh"
+extern "C" void radial(const double* s, const double* m, const double* a, int n, double* out)
+{
+    for (int i = 0; i < n; ++i) {
+        double y;
+        const double r = nb_sqrt_recip(s[i], nb_rsqrt_estimate(s[i]), y);
+        const double z = nb_recip_step(s[i], y * y);
+        const double t = (s[i] * s[i]) * r;
+        out[5 * i] = r;
+        out[5 * i + 1] = nb_quot(m[i], r, y);
+        out[5 * i + 2] = nb_quot(nb_quot(m[i], r, y), s[i], z);
+        out[5 * i + 3] = nb_recip_step(t, nb_recip_step(t, (z * z) * y));
+        out[5 * i + 4] = nb_quot(a[i], s[i], z);
+    }
+}
+extern "C" void ranges(const double* x, int n, int* out)
+{
+    for (int i = 0; i < n; ++i)
+        out[i] = nb_exp_in<-700, 700>(x[i]) | nb_pos_exp_in<-100, 100>(x[i]) << 1 |
+                 nb_near_ones(x[i]) << 2;
+}
+'''
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    d = tmp_path_factory.mktemp("rdiv")
+    src = d / "rdiv.cpp"
+    src.write_text(SRC)
+    so = d / "librdiv.so"
+    subprocess.run(["g++", "-O2", "-ffp-contract=off", "-mfma", "-fPIC", "-shared", "-I", CSRC,
+                    str(src), "-o", str(so)], check=True)
+    return ctypes.CDLL(str(so))
+
+
+def _near_ones(x):
+    return (x.view(np.uint64) >> np.uint64(32)) & np.uint64(0xfffff) == 0xfffff
+
+
+def _check(lib, s, m, a):
+    s, m, a = (np.ascontiguousarray(x, dtype=np.float64) for x in (s, m, a))
+    out = np.empty((len(s), 5))
+    p = [x.ctypes.data_as(ctypes.c_void_p) for x in (s, m, a)]
+    lib.radial(*p, ctypes.c_int(len(s)), out.ctypes.data_as(ctypes.c_void_p))
+    r = np.sqrt(s)
+    want = np.stack([r, m / r, (m / r) / s, 1.0 / ((s * s) * r), a / s], 1)
+    # the walk leaves divisors next to an all-ones significand to the operators (nb_near_ones)
+    ones = np.zeros(want.shape, bool)
+    ones[:] = _near_ones(s)[:, None]
+    ones[:, 3] |= _near_ones((s * s) * r)
+    bad = np.nonzero((out.view(np.uint64) != want.view(np.uint64)) & ~ones)
+    assert len(bad[0]) == 0, (bad[0][:5], bad[1][:5], out[bad][:5], want[bad][:5])
+
+
+def _random(rng, n, lo, hi):
+    x = np.ldexp(1.0 + rng.integers(0, 1 << 52, n) * 2.0 ** -52, rng.integers(lo, hi, n))
+    return x
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_random_operands(lib, seed):
+    rng = np.random.default_rng(seed)
+    n = 500_000
+    sign = rng.choice([-1.0, 1.0], n)
+    _check(lib, _random(rng, n, -100, 100), sign * _random(rng, n, -700, 700),
+           -sign * _random(rng, n, -700, 700))
+    _check(lib, _random(rng, n, -8, 12), _random(rng, n, -20, 4), sign * _random(rng, n, -40, 20))
+
+
+def test_operands_next_to_rounding_boundaries(lib):
+    """Roots whose square lies next to that of a midpoint of two doubles, and quotients a / s with
+    a = round(s q) for a midpoint q, a few ulps around each."""
+    rng = np.random.default_rng(9)
+    n = 200_000
+    k = rng.integers(1 << 52, 1 << 53, n, dtype=np.int64)
+    mid = [2 * int(v) + 1 for v in k[:20000]]
+    s = []
+    for v in mid:
+        sq = v * v                                  # (midpoint)^2, 107 or 108 bits
+        sh = sq.bit_length() - 53
+        for d in (-1, 0, 1, 2):
+            s.append(float((sq >> sh) + d) * 2.0 ** (sh - 107 + (sh & 1)))
+    s = np.array(s)
+    _check(lib, s, np.ones_like(s), np.ones_like(s))
+    s = _random(rng, n, -3, 3)
+    si = np.ldexp(s, 52 - np.frexp(s)[1] + 1).astype(np.int64)
+    a = np.array([float((int(x) * (2 * int(q) + 1) >> 53) + d)
+                  for x, q, d in zip(si, k, rng.integers(-1, 3, n))])
+    _check(lib, s, a, a)
+    # significands of all ones and of zeros, powers of two, neighbours of one
+    edge = np.array([1.0, 2.0, 4.0, 2.0 - 2.0 ** -52, 4.0 - 2.0 ** -51, 1.0 + 2.0 ** -52, 3.0,
+                     np.nextafter(0.25, 0), np.nextafter(0.5, 1)])
+    g = np.array(np.meshgrid(edge, edge, edge)).reshape(3, -1)
+    _check(lib, *g)
+
+
+def test_ranges(lib):
+    x = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, 2.0 ** -701, 2.0 ** -700, 2.0 ** 699,
+                  2.0 ** 700, -2.0 ** 699, 2.0 ** -101, 2.0 ** -100, 2.0 ** 99, 2.0 ** 100, -1.0])
+    out = np.empty(len(x), np.int32)
+    lib.ranges(x.ctypes.data_as(ctypes.c_void_p), ctypes.c_int(len(x)),
+               out.ctypes.data_as(ctypes.c_void_p))
+    ax = np.abs(x)
+    with np.errstate(invalid="ignore"):
+        want = ((ax >= 2.0 ** -700) & (ax < 2.0 ** 700)).astype(int) | \
+               (((x >= 2.0 ** -100) & (x < 2.0 ** 100)).astype(int) << 1)
+    assert (out & 3).tolist() == want.tolist()
+    x = np.array([2.0 - 2.0 ** -52, 2.0 - 2.0 ** -20, 2.0 - 2.0 ** -19, 1.0, 4.0 - 2.0 ** -51])
+    out = np.empty(len(x), np.int32)
+    lib.ranges(x.ctypes.data_as(ctypes.c_void_p), ctypes.c_int(len(x)),
+               out.ctypes.data_as(ctypes.c_void_p))
+    assert (out >> 2).tolist() == [1, 1, 0, 0, 1]
