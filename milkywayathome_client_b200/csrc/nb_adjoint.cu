@@ -393,8 +393,7 @@ void nb_launch_vjp(NbTreeBuffers& b, double* nodeBar, int capNodes, int maxDepth
     const int warps = (n + 31) / 32;
     cudaEventRecord(walkStart, s);
     // packed records from the (possibly restored) tree arrays
-    nb_launch_pack_walk(b.nodePM, b.nodeCrit, b.nodeLink, b.nodeQuad, b.walkRec, b.walkKids, capNodes,
-                        b.sc, s);
+    nb_launch_pack_walk(b, capNodes, false, s);
     k_walk_vjp<<<(warps * 32 + 127) / 128, 128, 0, s>>>(b.walkRec, b.sort.idxA, b.px, b.py, b.pz,
                                                         abar, xbar, nodeBar, wp, pot, b.sc);
     cudaEventRecord(walkEnd, s);

@@ -216,14 +216,14 @@ static void nb_free_nodes(NBodyCudaState* st)
     nb_drop_step_graph(st);             // its kernels hold the node arrays' addresses
     NbTreeBuffers& b = st->b;
     cudaFree(b.nodePM); cudaFree(b.nodeCrit); cudaFree(b.nodeLink); cudaFree(b.nodeQuad);
-    cudaFree(b.nodeDepth); cudaFree(b.parent); cudaFree(b.nchild); cudaFree(b.arrive);
+    cudaFree(b.nodeDepth); cudaFree(b.parent); cudaFree(b.pending); cudaFree(b.cellNode);
     cudaFree(b.nodeRange); b.nodeRange = nullptr;
     cudaFree(b.walkRec); b.walkRec = nullptr;
     cudaFree(b.walkKids); b.walkKids = nullptr;
     cudaFree(st->mx.groups);
-    cudaFree(st->mx.hi); cudaFree(st->mx.lo); cudaFree(st->mx.q32); cudaFree(st->mx.child8);
+    cudaFree(st->mx.hi); cudaFree(st->mx.lo); cudaFree(st->mx.q32);
     b.nodePM = nullptr; b.nodeCrit = nullptr; b.nodeLink = nullptr; b.nodeQuad = nullptr;
-    b.nodeDepth = b.parent = b.nchild = b.arrive = nullptr;
+    b.nodeDepth = b.parent = b.pending = b.cellNode = nullptr;
     int* stacks = st->mx.stacks;
     const int wb = st->mx.walkBlocks;
     st->mx = NbMixedBuffers{};
@@ -242,8 +242,8 @@ static NBodyCudaStatus nb_alloc_nodes(NBodyCudaState* st, int cap)
     NB_CHECK(nb_alloc(&b.nodeQuad, 6 * (size_t) cap));
     NB_CHECK(nb_alloc(&b.nodeDepth, cap));
     NB_CHECK(nb_alloc(&b.parent, cap));
-    NB_CHECK(nb_alloc(&b.nchild, cap));
-    NB_CHECK(nb_alloc(&b.arrive, cap));
+    NB_CHECK(nb_alloc(&b.pending, cap));
+    NB_CHECK(nb_alloc(&b.cellNode, cap));
     NB_CHECK(nb_alloc(&b.nodeRange, cap));
     NB_CHECK(nb_alloc(&b.walkRec, 3 * (size_t) cap));
     NB_CHECK(nb_alloc(&b.walkKids, 2 * (size_t) cap));
@@ -251,7 +251,6 @@ static NBodyCudaStatus nb_alloc_nodes(NBodyCudaState* st, int cap)
     NB_CHECK(nb_alloc(&st->mx.hi, cap));
     NB_CHECK(nb_alloc(&st->mx.lo, cap));
     NB_CHECK(nb_alloc(&st->mx.q32, 2 * (size_t) cap));
-    NB_CHECK(nb_alloc(&st->mx.child8, 2 * (size_t) cap));
     st->capNodes = cap;
     return NBODY_SUCCESS;
 }
@@ -510,10 +509,7 @@ static NBodyCudaStatus nb_force(const NBodyCudaCtx* ctx, NBodyCudaState* st, int
                 nb_launch_walk_mixed(b, st->mx, st->capNodes, wp, pot, st->counting != 0,
                                      st->numSMs, s);
             else
-                nb_launch_walk_fp64(b.nodePM, b.nodeCrit, b.nodeLink, b.nodeQuad, b.sort.idxA, b.px,
-                                    b.py, b.pz, b.ax, b.ay, b.az, b.vx, b.vy, b.vz, wp, pot, b.sc,
-                                    st->counting != 0, s, b.walkRec, b.walkKids, st->capNodes, nullptr,
-                                    form);
+                nb_launch_walk_fp64(b, st->capNodes, wp, pot, st->counting != 0, s, nullptr, form);
             rec(st->ev1);
         }
         rec(st->evE);
@@ -2105,9 +2101,8 @@ static int nb_batch_enqueue(NBodyCudaBatch* bt, const NBodyCudaCtx* ctx, int dri
         nb_launch_walk_mixed(b, st->mx, st->capNodes, wp, pot, false, st->numSMs, s, &f);
         launches += 3;
     } else {
-        nb_launch_walk_fp64(b.nodePM, b.nodeCrit, b.nodeLink, b.nodeQuad, b.sort.idxA, b.px, b.py,
-                            b.pz, b.ax, b.ay, b.az, b.vx, b.vy, b.vz, wp, pot, b.sc, false, s,
-                            b.walkRec, b.walkKids, st->capNodes, &f, st->walkForm > 0 ? st->walkForm : 0);
+        nb_launch_walk_fp64(b, st->capNodes, wp, pot, false, s, &f,
+                            st->walkForm > 0 ? st->walkForm : 0);
         launches += 1;
     }
     cudaEventRecord(st->ev1, s);

@@ -265,7 +265,8 @@ __global__ void k_b_emit_bodies(const double* __restrict__ px, const double* __r
 
 // Cells owned by boundary a (as k_emit_cells), geometry from the dwarf's root size; the
 // depth-0 cell of a dwarf is its root and records the dwarf's node range.
-__global__ void k_b_emit_cells(const long long* __restrict__ gx, const long long* __restrict__ gy,
+__global__ void k_b_emit_cells(const unsigned long long* __restrict__ key,
+                               const long long* __restrict__ gx, const long long* __restrict__ gy,
                                const long long* __restrict__ gz, const int* __restrict__ delta,
                                const int* __restrict__ cum, const int* __restrict__ bodyDwarf,
                                NbDwarfDev* __restrict__ dw, double4* __restrict__ nodePM,
@@ -292,7 +293,7 @@ __global__ void k_b_emit_cells(const long long* __restrict__ gx, const long long
         }
         for (int D = dPrev + 1; D <= dHere; ++D) {
             const int p = a + cellsBefore + (D - dPrev - 1);
-            const int last = nb_range_end(gx, gy, gz, a, D, dEnd);
+            const int last = nb_range_end(key, gx, gy, gz, a, D, dEnd);
             const int next = last + nb_b_cells_before_body(cum, last, n) + 1;
             nodeRange[p] = make_int2(a, last);
             nodePM[p] = make_double4(cx, cy, cz, 0.0);
@@ -311,10 +312,11 @@ __global__ void k_b_emit_cells(const long long* __restrict__ gx, const long long
     }
 }
 
-// Parents (-1 for every dwarf's root) and child counts from Next().
+// Parents (-1 for every dwarf's root) and child lists from Next().
 __global__ void k_b_link_children(const int2* __restrict__ nodeLink, const int* __restrict__ nodeDepth,
-                                  int* __restrict__ parent, int* __restrict__ nchild,
-                                  int* __restrict__ arrive, NbScalars* __restrict__ sc)
+                                  const int2* __restrict__ nodeRange, int* __restrict__ parent,
+                                  int* __restrict__ pending, int* __restrict__ cellNode,
+                                  int4* __restrict__ kids, NbScalars* __restrict__ sc)
 {
     if (nb_failed(sc)) return;
     const int nNodes = sc->nNodes;
@@ -322,90 +324,31 @@ __global__ void k_b_link_children(const int2* __restrict__ nodeLink, const int* 
         const int2 l = nodeLink[c];
         if (l.y >= 0) continue;            // body
         if (nodeDepth[c] == 0) parent[c] = -1;
-        int k = c + 1, count = 0;
-        while (k < l.x) {
-            parent[k] = c;
-            ++count;
-            k = nodeLink[k].x;
-        }
-        nchild[c] = count;
-        arrive[c] = 0;
+        nb_link_cell(c, l, c - nodeRange[c].x, nodeLink, parent, pending, cellNode, kids);
     }
 }
 
 // Bottom-up moments (as k_moments) with the dwarf's root size.
-__global__ void k_b_moments(double4* __restrict__ nodePM, double* __restrict__ nodeCrit,
-                            const int2* __restrict__ nodeLink, const int* __restrict__ nodeDepth,
-                            double* __restrict__ nodeQuad, const int* __restrict__ parent,
-                            const int* __restrict__ nchild, int* __restrict__ arrive,
-                            const int* __restrict__ bodyNode, const int* __restrict__ bodyDwarf,
-                            NbDwarfDev* __restrict__ dw, int criterion, double theta, int useQuad,
-                            int n, NbScalars* __restrict__ sc)
+__global__ void __launch_bounds__(128, 4)
+k_b_moments(double4* nodePM, double* nodeCrit, const int2* nodeLink, const int* nodeDepth,
+            const int2* nodeRange, double* nodeQuad, const int* __restrict__ parent, int* pending,
+            const int* __restrict__ cellNode, const int4* kids, const int* __restrict__ bodyDwarf,
+            NbDwarfDev* dw, int criterion, double theta, int useQuad, NbScalars* sc)
 {
     if (nb_failed(sc)) return;
+    const int nCells = sc->nCells;
     int structErr = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int dwi = bodyDwarf[i];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nCells; i += gridDim.x * blockDim.x) {
+        if (cellNode[i] < 0) continue;
+        const int dwi = bodyDwarf[nodeRange[cellNode[i]].x];
         const double rsize = dw[dwi].rsize;
-        int c = parent[bodyNode[i]];
-        while (c >= 0) {
-            __threadfence();
-            if (atomicAdd(&arrive[c], 1) != nchild[c] - 1) break;   // not the last child
-            __threadfence();
-            const int end = __ldcg(&nodeLink[c].x);
-            const double4 geo = nb_ld_pm(&nodePM[c]);
-            double M = 0.0, cmx = 0.0, cmy = 0.0, cmz = 0.0;
-            for (int k = c + 1; k < end; k = __ldcg(&nodeLink[k].x)) {
-                const double4 q = nb_ld_pm(&nodePM[k]);
-                M = M + q.w;
-                cmx = cmx + q.w * q.x;
-                cmy = cmy + q.w * q.y;
-                cmz = cmz + q.w * q.z;
-            }
-            if (M > 0.0) { cmx = cmx / M; cmy = cmy / M; cmz = cmz / M; }
-            else { cmx = geo.x; cmy = geo.y; cmz = geo.z; }
-            const int D = __ldcg(&nodeDepth[c]);
-            double psize = rsize;
-            for (int d = 0; d < D; ++d) psize *= 0.5;
-            const double h = 0.5 * psize;
-            if (cmx < geo.x - h || cmx > geo.x + h || cmy < geo.y - h || cmy > geo.y + h ||
-                cmz < geo.z - h || cmz > geo.z + h) {
+        nb_bottom_up(i, cellNode, parent, pending, [&](int c) {
+            if (nb_cell_moments(c, nodePM, nodeCrit, nodeLink, nodeDepth, nodeRange, nodeQuad, kids,
+                                rsize, criterion, theta, useQuad)) {
                 structErr = 1;
                 atomicOr(&dw[dwi].status, NBODY_TREE_STRUCTURE_ERROR);
             }
-            nodeCrit[c] = nb_find_rcrit2(criterion, theta, rsize, geo.x, geo.y, geo.z,
-                                         cmx, cmy, cmz, psize);
-            if (useQuad) {
-                double qxx = 0.0, qxy = 0.0, qxz = 0.0, qyy = 0.0, qyz = 0.0, qzz = 0.0;
-                for (int k = c + 1; k < end; k = __ldcg(&nodeLink[k].x)) {
-                    const double4 q = nb_ld_pm(&nodePM[k]);
-                    const double dx = q.x - cmx, dy = q.y - cmy, dz = q.z - cmz;
-                    const double drsq = dz * dz + (dy * dy + dx * dx);
-                    const double mq = q.w;
-                    double txx = mq * (3.0 * (dx * dx) - drsq);
-                    double txy = mq * (3.0 * (dx * dy));
-                    double txz = mq * (3.0 * (dx * dz));
-                    double tyy = mq * (3.0 * (dy * dy) - drsq);
-                    double tyz = mq * (3.0 * (dy * dz));
-                    double tzz = mq * (3.0 * (dz * dz) - drsq);
-                    if (__ldcg(&nodeLink[k].y) < 0) {
-                        const double* Q = nodeQuad + 6 * (size_t) k;
-                        txx = txx + __ldcg(Q + 0); txy = txy + __ldcg(Q + 1); txz = txz + __ldcg(Q + 2);
-                        tyy = tyy + __ldcg(Q + 3); tyz = tyz + __ldcg(Q + 4); tzz = tzz + __ldcg(Q + 5);
-                    }
-                    qxx = qxx + txx; qxy = qxy + txy; qxz = qxz + txz;
-                    qyy = qyy + tyy; qyz = qyz + tyz; qzz = qzz + tzz;
-                }
-                double* Q = nodeQuad + 6 * (size_t) c;
-                Q[0] = qxx; Q[1] = qxy; Q[2] = qxz; Q[3] = qyy; Q[4] = qyz; Q[5] = qzz;
-            } else {
-                // no quadrupoles: the record reads as zero (as the restated CPU tree does)
-                double* Q = nodeQuad + 6 * (size_t) c;
-                for (int k = 0; k < 6; ++k) Q[k] = 0.0;
-            }
-            nodePM[c] = make_double4(cmx, cmy, cmz, M);
-            c = parent[c];
-        }
+        });
     }
     if (structErr) nb_raise(sc, NBODY_TREE_STRUCTURE_ERROR);
 }
@@ -455,15 +398,14 @@ int nb_build_forest(NbTreeBuffers& b, const NbForest& f, int n, int capNodes, in
     k_b_emit_bodies<<<g, T, 0, s>>>(b.px, b.py, b.pz, b.mass, b.sort.idxA, b.delta, b.cum,
                                     b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.bodyNode,
                                     b.nodeRange, n, b.sc);
-    k_b_emit_cells<<<g, T, 0, s>>>(b.gx, b.gy, b.gz, b.delta, b.cum, f.bodyDwarf, f.dwarfs,
+    k_b_emit_cells<<<g, T, 0, s>>>(b.sort.keyA, b.gx, b.gy, b.gz, b.delta, b.cum, f.bodyDwarf, f.dwarfs,
                                    b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.nodeRange, n,
                                    b.sc);
-    k_b_link_children<<<nb_b_grid(capNodes, T, 1 << 20), T, 0, s>>>(b.nodeLink, b.nodeDepth,
-                                                                    b.parent, b.nchild, b.arrive,
-                                                                    b.sc);
-    k_b_moments<<<g, T, 0, s>>>(b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.nodeQuad,
-                                b.parent, b.nchild, b.arrive, b.bodyNode, f.bodyDwarf, f.dwarfs,
-                                criterion, theta, useQuad, n, b.sc);
+    k_b_link_children<<<nb_b_grid(capNodes, T, 1 << 20), T, 0, s>>>(
+        b.nodeLink, b.nodeDepth, b.nodeRange, b.parent, b.pending, b.cellNode, b.walkKids, b.sc);
+    k_b_moments<<<nb_b_grid(n, 128, 1 << 20), 128, 0, s>>>(
+        b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.nodeRange, b.nodeQuad, b.parent, b.pending,
+        b.cellNode, b.walkKids, f.bodyDwarf, f.dwarfs, criterion, theta, useQuad, b.sc);
     launches += 5;
     nb_count_launch(launches - 53);       // the sort and the scan count their own
     return launches;

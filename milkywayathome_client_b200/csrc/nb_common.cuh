@@ -282,10 +282,13 @@ struct NbTreeBuffers {
     long long *gx, *gy, *gz;
     int *delta, *cum, *scanTmp, *bodyNode;
     double4* nodePM; double* nodeCrit; int2* nodeLink; double* nodeQuad;
-    int *nodeDepth, *parent, *nchild, *arrive;
+    int *nodeDepth;
+    int *parent;       // of every cell (bodies' entries unused)
+    int *pending;      // child cells a cell's moments still wait for
+    int *cellNode;     // the node of every cell slot (complemented: it has child cells)
     int2* nodeRange;   // first and last sorted body of every node's subtree
     double4* walkRec;  // 3 per node: the FP64 walk's packed node records
-    int4* walkKids;    // 2 per node: a cell's children, up to 8 (-1: none)
+    int4* walkKids;    // 2 per cell, by slot: its children in octant order, up to 8 (-1: none)
     NbScalars* sc;
 };
 
@@ -294,7 +297,6 @@ struct NbMixedBuffers {
     float4* hi;    // {hi.x, hi.y, hi.z, rcrit2 (-inf for bodies)}
     float4* lo;    // {lo.x, lo.y, lo.z, mass}
     float4* q32;   // 2 per node: {xx, xy, xz, yy}, {yz, zz, 0, 0}
-    int4* child8;  // 2 per node: up to 8 child indices of a cell (-1 = none)
     int* stacks;   // per resident warp: the group walk's depth-first stack
     int2* groups;  // walk groups: first sorted body, body count (<= 32)
     int walkBlocks;
@@ -305,21 +307,16 @@ struct NbMixedBuffers {
 int nb_mixed_walk_blocks(int numSMs, int listCap = 0, int groupMax = 32);
 size_t nb_mixed_stack_ints(int blocks);
 
-// The FP64 walks' packed node records (3 double4 per node) from the tree arrays.
-void nb_launch_pack_walk(const double4* nodePM, const double* nodeCrit, const int2* nodeLink,
-                         const double* nodeQuad, double4* rec, int4* kids, int capNodes,
-                         const NbScalars* sc, cudaStream_t s);
+// The FP64 walks' packed node records (3 double4 per node) from the tree arrays.  slots: cells
+// carry their slot in walkKids (the force adjoint's restored trees have none, and no use for it).
+void nb_launch_pack_walk(const NbTreeBuffers& b, int capNodes, bool slots, cudaStream_t s);
 
 // The walks (forest != nullptr: one tree per dwarf, see NbForest).  form: the FP64 walk's
 // form, 0 the team walk where nb_walk_team(n) (else as 1), 1 the walk per lane, 2 per lane with
 // the next record loaded early.
 bool nb_walk_team(int n);
-void nb_launch_walk_fp64(const double4* nodePM, const double* nodeCrit, const int2* nodeLink,
-                         const double* nodeQuad, const unsigned* order, const double* px,
-                         const double* py, const double* pz, double* ax, double* ay, double* az,
-                         double* vx, double* vy, double* vz, const NbWalkParams& wp,
-                         const NbPot& pot, NbScalars* sc, bool count, cudaStream_t s,
-                         double4* walkRec, int4* walkKids, int capNodes,
+void nb_launch_walk_fp64(const NbTreeBuffers& b, int capNodes, const NbWalkParams& wp,
+                         const NbPot& pot, bool count, cudaStream_t s,
                          const NbForest* forest = nullptr, int form = 0);
 void nb_launch_walk_mixed(const NbTreeBuffers& b, const NbMixedBuffers& m, int capNodes,
                           const NbWalkParams& wp, const NbPot& pot, bool count, int numSMs,

@@ -20,6 +20,7 @@
 // code, compiled with -fmad=false so the shared epilogue keeps the reference's rounding).
 #include "nb_common.cuh"
 #include "nb_potential.cuh"
+#include "nb_tree_util.cuh"
 
 
 __device__ __forceinline__ void nb_split(double v, float& hi, float& lo)
@@ -34,8 +35,7 @@ template <bool FOREST>
 __global__ void k_pack_f32(const double4* __restrict__ nodePM, const double* __restrict__ nodeCrit,
                            const int2* __restrict__ nodeLink, const double* __restrict__ nodeQuad,
                            float4* __restrict__ nodeHi, float4* __restrict__ nodeLo,
-                           float4* __restrict__ nodeQ32, int4* __restrict__ child8,
-                           const int2* __restrict__ nodeRange, const NbScalars* __restrict__ sc,
+                           float4* __restrict__ nodeQ32, const int2* __restrict__ nodeRange, const NbScalars* __restrict__ sc,
                            NbForest forest)
 {
     if (nb_failed(sc)) return;
@@ -60,13 +60,6 @@ __global__ void k_pack_f32(const double4* __restrict__ nodePM, const double* __r
             // densely by slot, and lo.w carries the slot (the mass is in the slot's record)
             const int c = k - nodeRange[k].x;
             nodeLo[k] = make_float4(lx, ly, lz, __int_as_float(c));
-            // the children of a cell: k+1, then Next() up to Next(k) (threadTree order)
-            int ch[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
-            const int stop = nodeLink[k].x;
-            int kc = k + 1;
-            for (int m = 0; m < 8 && kc < stop; ++m) { ch[m] = kc; kc = nodeLink[kc].x; }
-            child8[2 * (size_t) c] = make_int4(ch[0], ch[1], ch[2], ch[3]);
-            child8[2 * (size_t) c + 1] = make_int4(ch[4], ch[5], ch[6], ch[7]);
             const double* Q = nodeQuad + 6 * (size_t) k;
             nodeQ32[2 * (size_t) c] = make_float4(__double2float_rn(Q[0]), __double2float_rn(Q[1]),
                                                   __double2float_rn(Q[2]), __double2float_rn(Q[3]));
@@ -220,16 +213,38 @@ __device__ __forceinline__ void nb_eval_cells(const CellList<LIST_CAP>& list, in
 // 72 % of the lanes on a 1M-body Plummer dwarf at theta = 0.5) and cut the interaction work
 // by 17 %, the most expensive group staying within 1.5 x the mean.
 // With a forest every dwarf's root counts as a root.
-__device__ __forceinline__ void nb_put_runs(int2* __restrict__ groups, NbScalars* __restrict__ sc,
-                                            int first, int count, int G)
+//
+// One thread lays out a cell: it counts the groups first and takes their numbers with one atomic
+// (an atomic per group, up to a few hundred one after another for a large cell, was most of the
+// kernel: 115 -> 27 us at 1,048,576 bodies, 38 -> 8 at 20,000).
+template <typename Put>
+__device__ __forceinline__ void nb_cell_groups(const int2 (&range)[8], int G, int T, Put put)
 {
-    for (int o = 0; o < count; o += G)
-        groups[atomicAdd(&sc->nGroups, 1)] = make_int2(first + o, min(G, count - o));
+    int gFirst = -1, gCount = 0;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        const int ck = range[m].y - range[m].x + 1;
+        if (ck <= 0) continue;                               // past the last child
+        if (ck > G) {
+            if (gCount) put(gFirst, gCount);
+            gCount = 0;
+            if (ck <= T)                                     // else laid out by its own thread
+                for (int o = 0; o < ck; o += G) put(range[m].x + o, min(G, ck - o));
+            continue;
+        }
+        if (gCount && gCount + ck > G) {
+            put(gFirst, gCount);
+            gCount = 0;
+        }
+        if (!gCount) gFirst = range[m].x;
+        gCount += ck;
+    }
+    if (gCount) put(gFirst, gCount);
 }
 
 __global__ void k_groups(const int2* __restrict__ nodeLink, const int2* __restrict__ nodeRange,
-                         int2* __restrict__ groups, int n, NbScalars* __restrict__ sc, int G,
-                         NbForest forest)
+                         const int4* __restrict__ kids, int2* __restrict__ groups, int n,
+                         NbScalars* __restrict__ sc, int G, NbForest forest)
 {
     if (nb_failed(sc)) return;
     const int nNodes = sc->nNodes, m = sc->nTree;
@@ -237,34 +252,29 @@ __global__ void k_groups(const int2* __restrict__ nodeLink, const int2* __restri
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int stride = gridDim.x * blockDim.x;
     for (int c = tid; c < nNodes; c += stride) {
-        const int2 l = nodeLink[c];
-        if (l.y >= 0) continue;                              // bodies are handled by parents
         const int2 r = nodeRange[c];
         const int cnt = r.y - r.x + 1;
+        if (cnt <= 1 && c != 0) continue;                    // bodies are handled by parents
+        if (nodeLink[c].y >= 0) continue;
         if (cnt <= T) {
-            const bool root = forest.dwarfs ? c == forest.dwarfs[forest.bodyDwarf[r.x]].rootNode
-                                            : c == 0;
-            if (root && cnt > 0) nb_put_runs(groups, sc, r.x, cnt, G);
+            const bool root = cnt > 0 && (forest.dwarfs ? c == forest.dwarfs[forest.bodyDwarf[r.x]].rootNode
+                                                        : c == 0);
+            if (root) {
+                int at = atomicAdd(&sc->nGroups, (cnt + G - 1) / G);
+                for (int o = 0; o < cnt; o += G) groups[at++] = make_int2(r.x + o, min(G, cnt - o));
+            }
             continue;
         }
-        int gFirst = -1, gCount = 0;
-        for (int k = c + 1; k < l.x; k = nodeLink[k].x) {
-            const int2 rk = nodeRange[k];
-            const int ck = rk.y - rk.x + 1;
-            if (ck > G) {
-                if (gCount) groups[atomicAdd(&sc->nGroups, 1)] = make_int2(gFirst, gCount);
-                gCount = 0;
-                if (ck <= T) nb_put_runs(groups, sc, rk.x, ck, G);   // else its own thread
-                continue;
-            }
-            if (gCount && gCount + ck > G) {
-                groups[atomicAdd(&sc->nGroups, 1)] = make_int2(gFirst, gCount);
-                gCount = 0;
-            }
-            if (!gCount) gFirst = rk.x;
-            gCount += ck;
-        }
-        if (gCount) groups[atomicAdd(&sc->nGroups, 1)] = make_int2(gFirst, gCount);
+        int k[8];
+        nb_load_kids(kids, c - r.x, k);
+        int2 range[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) range[q] = k[q] >= 0 ? nodeRange[k[q]] : make_int2(0, -1);
+        int count = 0;
+        nb_cell_groups(range, G, T, [&](int, int) { ++count; });
+        if (!count) continue;
+        int at = atomicAdd(&sc->nGroups, count);
+        nb_cell_groups(range, G, T, [&](int first, int num) { groups[at++] = make_int2(first, num); });
     }
     for (int t = tid; m + G * t < n; t += stride)
         groups[atomicAdd(&sc->nGroups, 1)] = make_int2(m + G * t, min(G, n - m - G * t));
@@ -549,11 +559,11 @@ static void nb_walk_mixed_launch(const NbTreeBuffers& b, const NbMixedBuffers& m
 {
     if (m.exact)
         k_walk_mixed<COUNT, FOREST, LC, BPL, true><<<blocks, GROUP_THREADS, 0, s>>>(
-            m.hi, m.lo, m.q32, m.child8, b.nodePM, b.sort.idxA, b.px, b.py, b.pz, b.mass, b.ax,
+            m.hi, m.lo, m.q32, b.walkKids, b.nodePM, b.sort.idxA, b.px, b.py, b.pz, b.mass, b.ax,
             b.ay, b.az, m.stacks, m.groups, wp, b.sc, f);
     else
         k_walk_mixed<COUNT, FOREST, LC, BPL, false><<<blocks, GROUP_THREADS, 0, s>>>(
-            m.hi, m.lo, m.q32, m.child8, b.nodePM, b.sort.idxA, b.px, b.py, b.pz, b.mass, b.ax,
+            m.hi, m.lo, m.q32, b.walkKids, b.nodePM, b.sort.idxA, b.px, b.py, b.pz, b.mass, b.ax,
             b.ay, b.az, m.stacks, m.groups, wp, b.sc, f);
 }
 
@@ -590,12 +600,12 @@ void nb_launch_walk_mixed(const NbTreeBuffers& b, const NbMixedBuffers& m, int c
     const int g = min((capNodes + 255) / 256, numSMs * 16);
     if (forest)
         k_pack_f32<true><<<g, 256, 0, s>>>(b.nodePM, b.nodeCrit, b.nodeLink, b.nodeQuad, m.hi, m.lo,
-                                           m.q32, m.child8, b.nodeRange, b.sc, f);
+                                           m.q32, b.nodeRange, b.sc, f);
     else
         k_pack_f32<false><<<g, 256, 0, s>>>(b.nodePM, b.nodeCrit, b.nodeLink, b.nodeQuad, m.hi, m.lo,
-                                            m.q32, m.child8, b.nodeRange, b.sc, f);
+                                            m.q32, b.nodeRange, b.sc, f);
     const int G = m.groupMax >= 1 && m.groupMax <= 64 ? m.groupMax : 32;
-    k_groups<<<g, 256, 0, s>>>(b.nodeLink, b.nodeRange, m.groups, wp.n, b.sc, G, f);
+    k_groups<<<g, 256, 0, s>>>(b.nodeLink, b.nodeRange, b.walkKids, m.groups, wp.n, b.sc, G, f);
     nb_count_launch(2);
     if (wp.n <= 0) return;
     const int blocks = m.walkBlocks;

@@ -242,7 +242,8 @@ __global__ void k_emit_bodies(const double* __restrict__ px, const double* __res
 // Cells owned by boundary a: depths (delta_{a-1}, delta_a].  Writes the geometric centre
 // (nbInitMidpoint/calcOffset, :226-239: c += 0.25 * (+-size) level by level from the
 // origin) into nodePM.xyz until the moment pass replaces it by the centre of mass.
-__global__ void k_emit_cells(const long long* __restrict__ gx, const long long* __restrict__ gy,
+__global__ void k_emit_cells(const unsigned long long* __restrict__ key,
+                             const long long* __restrict__ gx, const long long* __restrict__ gy,
                              const long long* __restrict__ gz, const int* __restrict__ delta,
                              const int* __restrict__ cum, double4* __restrict__ nodePM,
                              double* __restrict__ nodeCrit, int2* __restrict__ nodeLink,
@@ -276,7 +277,7 @@ __global__ void k_emit_cells(const long long* __restrict__ gx, const long long* 
             int next, last;
             if (m <= 1) { next = m + 1; last = m - 1; }
             else {
-                last = nb_range_end(gx, gy, gz, a, D, m);
+                last = nb_range_end(key, gx, gy, gz, a, D, m);
                 next = last + nb_cells_before_body(cum, last, m) + 1;
             }
             nodeRange[p] = make_int2(a, last);
@@ -301,9 +302,10 @@ __global__ void k_emit_cells(const long long* __restrict__ gx, const long long* 
     }
 }
 
-// Parent pointers and child counts from Next() (children of cell c: c+1, then Next()).
-__global__ void k_link_children(const int2* __restrict__ nodeLink, int* __restrict__ parent,
-                                int* __restrict__ nchild, int* __restrict__ arrive,
+// Parent pointers and child lists from Next().
+__global__ void k_link_children(const int2* __restrict__ nodeLink, const int2* __restrict__ nodeRange,
+                                int* __restrict__ parent, int* __restrict__ pending,
+                                int* __restrict__ cellNode, int4* __restrict__ kids,
                                 NbScalars* __restrict__ sc)
 {
     if (nb_failed(sc)) return;
@@ -312,93 +314,29 @@ __global__ void k_link_children(const int2* __restrict__ nodeLink, int* __restri
         if (c == 0) parent[0] = -1;
         const int2 l = nodeLink[c];
         if (l.y >= 0) continue;            // body
-        int k = c + 1, count = 0;
-        while (k < l.x) {
-            parent[k] = c;
-            ++count;
-            k = nodeLink[k].x;
-        }
-        nchild[c] = count;
-        arrive[c] = 0;
+        nb_link_cell(c, l, c - nodeRange[c].x, nodeLink, parent, pending, cellNode, kids);
     }
 }
 
 // ---------------------------------------------------------------------------------
 // 6. moments, bottom-up
 // ---------------------------------------------------------------------------------
-__global__ void k_moments(double4* __restrict__ nodePM, double* __restrict__ nodeCrit,
-                          const int2* __restrict__ nodeLink, const int* __restrict__ nodeDepth,
-                          double* __restrict__ nodeQuad, const int* __restrict__ parent,
-                          const int* __restrict__ nchild, int* __restrict__ arrive,
-                          const int* __restrict__ bodyNode, int criterion, double theta,
-                          int useQuad, NbScalars* __restrict__ sc)
+// One thread per cell, from the cells without child cells up (nb_bottom_up).
+__global__ void __launch_bounds__(128, 4)
+k_moments(double4* nodePM, double* nodeCrit, const int2* nodeLink, const int* nodeDepth,
+          const int2* nodeRange, double* nodeQuad, const int* __restrict__ parent, int* pending,
+          const int* __restrict__ cellNode, const int4* kids, int criterion, double theta,
+          int useQuad, NbScalars* sc)
 {
     if (nb_failed(sc)) return;
-    const int m = sc->nTree;
+    const int nCells = sc->nCells;
     const double rsize = sc->rsize;
     int structErr = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-        int c = parent[bodyNode[i]];
-        while (c >= 0) {
-            __threadfence();
-            if (atomicAdd(&arrive[c], 1) != nchild[c] - 1) break;   // not the last child
-            __threadfence();
-            const int end = __ldcg(&nodeLink[c].x);
-            const double4 geo = nb_ld_pm(&nodePM[c]);
-            // hackCofM (:394-424)
-            double M = 0.0, cmx = 0.0, cmy = 0.0, cmz = 0.0;
-            for (int k = c + 1; k < end; k = __ldcg(&nodeLink[k].x)) {
-                const double4 q = nb_ld_pm(&nodePM[k]);
-                M = M + q.w;
-                cmx = cmx + q.w * q.x;
-                cmy = cmy + q.w * q.y;
-                cmz = cmz + q.w * q.z;
-            }
-            if (M > 0.0) { cmx = cmx / M; cmy = cmy / M; cmz = cmz / M; }
-            else { cmx = geo.x; cmy = geo.y; cmz = geo.z; }
-            const int D = __ldcg(&nodeDepth[c]);
-            double psize = rsize;
-            for (int d = 0; d < D; ++d) psize *= 0.5;
-            // nbCheckTreeStructure (:345-380)
-            const double h = 0.5 * psize;
-            if (cmx < geo.x - h || cmx > geo.x + h || cmy < geo.y - h || cmy > geo.y + h ||
-                cmz < geo.z - h || cmz > geo.z + h)
-                structErr = 1;
-            nodeCrit[c] = nb_find_rcrit2(criterion, theta, rsize, geo.x, geo.y, geo.z,
-                                         cmx, cmy, cmz, psize);
-            if (useQuad) {
-                // hackQuad (:70-121), children in octant order
-                double qxx = 0.0, qxy = 0.0, qxz = 0.0, qyy = 0.0, qyz = 0.0, qzz = 0.0;
-                for (int k = c + 1; k < end; k = __ldcg(&nodeLink[k].x)) {
-                    const double4 q = nb_ld_pm(&nodePM[k]);
-                    const double dx = q.x - cmx, dy = q.y - cmy, dz = q.z - cmz;
-                    const double drsq = dz * dz + (dy * dy + dx * dx);
-                    const double mq = q.w;
-                    double txx = mq * (3.0 * (dx * dx) - drsq);
-                    double txy = mq * (3.0 * (dx * dy));
-                    double txz = mq * (3.0 * (dx * dz));
-                    double tyy = mq * (3.0 * (dy * dy) - drsq);
-                    double tyz = mq * (3.0 * (dy * dz));
-                    double tzz = mq * (3.0 * (dz * dz) - drsq);
-                    if (__ldcg(&nodeLink[k].y) < 0) {
-                        const double* Q = nodeQuad + 6 * (size_t) k;
-                        txx = txx + __ldcg(Q + 0); txy = txy + __ldcg(Q + 1); txz = txz + __ldcg(Q + 2);
-                        tyy = tyy + __ldcg(Q + 3); tyz = tyz + __ldcg(Q + 4); tzz = tzz + __ldcg(Q + 5);
-                    }
-                    qxx = qxx + txx; qxy = qxy + txy; qxz = qxz + txz;
-                    qyy = qyy + tyy; qyz = qyz + tyz; qzz = qzz + tzz;
-                }
-                double* Q = nodeQuad + 6 * (size_t) c;
-                Q[0] = qxx; Q[1] = qxy; Q[2] = qxz; Q[3] = qyy; Q[4] = qyz; Q[5] = qzz;
-            } else {
-                // no quadrupoles: the record reads as zero (as the restated CPU tree does)
-                double* Q = nodeQuad + 6 * (size_t) c;
-                for (int k = 0; k < 6; ++k) Q[k] = 0.0;
-            }
-            nodePM[c] = make_double4(cmx, cmy, cmz, M);
-            c = parent[c];
-        }
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nCells; i += gridDim.x * blockDim.x)
+        nb_bottom_up(i, cellNode, parent, pending, [&](int c) {
+            structErr |= nb_cell_moments(c, nodePM, nodeCrit, nodeLink, nodeDepth, nodeRange,
+                                         nodeQuad, kids, rsize, criterion, theta, useQuad);
+        });
     if (structErr) nb_raise(sc, NBODY_TREE_STRUCTURE_ERROR);
 }
 
@@ -443,7 +381,7 @@ void nb_build_tree(NbTreeBuffers& b, int n, int criterion, double theta, int use
     k_count_nodes<<<1, 1, 0, s>>>(b.cum, b.sc);
     k_emit_bodies<<<g, T, 0, s>>>(b.px, b.py, b.pz, b.mass, b.sort.idxA, b.delta, b.cum, b.nodePM,
                                   b.nodeCrit, b.nodeLink, b.nodeDepth, b.bodyNode, b.nodeRange, b.sc);
-    k_emit_cells<<<g, T, 0, s>>>(b.gx, b.gy, b.gz, b.delta, b.cum, b.nodePM, b.nodeCrit,
+    k_emit_cells<<<g, T, 0, s>>>(b.sort.keyA, b.gx, b.gy, b.gz, b.delta, b.cum, b.nodePM, b.nodeCrit,
                                  b.nodeLink, b.nodeDepth, b.nodeQuad, b.nodeRange, criterion, theta,
                                  b.sc);
     nb_count_launch(3);
@@ -454,10 +392,13 @@ void nb_link_and_moments(NbTreeBuffers& b, int n, int capNodes, int criterion, d
 {
     const int T = 256;
     const int gNodes = nb_grid_for(capNodes, T, 1 << 20);
-    const int g = nb_grid_for(n, T, 1 << 20);
-    k_link_children<<<gNodes, T, 0, s>>>(b.nodeLink, b.parent, b.nchild, b.arrive, b.sc);
-    k_moments<<<g, T, 0, s>>>(b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.nodeQuad, b.parent,
-                              b.nchild, b.arrive, b.bodyNode, criterion, theta, useQuad, b.sc);
+    k_link_children<<<gNodes, T, 0, s>>>(b.nodeLink, b.nodeRange, b.parent, b.pending, b.cellNode,
+                                         b.walkKids, b.sc);
+    // a cell parts at least two bodies (or is the root), but chains of single-child cells make
+    // more of them than bodies now and then: the loop takes any number
+    k_moments<<<nb_grid_for(n, 128, 1 << 20), 128, 0, s>>>(
+        b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.nodeRange, b.nodeQuad, b.parent, b.pending,
+        b.cellNode, b.walkKids, criterion, theta, useQuad, b.sc);
     nb_count_launch(2);
 }
 

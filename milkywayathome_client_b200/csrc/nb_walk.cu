@@ -19,34 +19,28 @@ constexpr int WALK_THREADS = 128;
 // FOREST: the nodes hold one tree per dwarf (batched dwarfs); each lane walks its own
 // dwarf's tree, [rootNode, rootEnd), with that dwarf's softening and time step.
 // The walk reads one packed record per node (k_pack_walk): 96 bytes, three double4 --
-// {CoM, mass}, {rcrit2, Next and body index as one 64-bit word, Qxx, Qxy},
-// {Qxz, Qyy, Qyz, Qzz} -- so a visit touches one record instead of four arrays -- and, for the
-// team walk, every cell's children (8 node numbers, -1 past the last).
+// {CoM, mass}, {rcrit2, Next and, as one 64-bit word with it, the body index or the complement of
+// the cell's slot, Qxx, Qxy}, {Qxz, Qyy, Qyz, Qzz} -- so a visit touches one record instead of four
+// arrays.  (128-byte records that also held the children were measured: the per-lane walk of 1M
+// bodies went from 28.9 to 37.6 ms.)
 __global__ void k_pack_walk(const double4* __restrict__ nodePM, const double* __restrict__ nodeCrit,
-                            const int2* __restrict__ nodeLink, const double* __restrict__ nodeQuad,
-                            double4* __restrict__ rec, int4* __restrict__ kids,
+                            const int2* __restrict__ nodeLink, const int2* __restrict__ nodeRange,
+                            const double* __restrict__ nodeQuad, double4* __restrict__ rec,
                             const NbScalars* __restrict__ sc)
 {
     if (nb_failed(sc)) return;
     const int nNodes = sc->nNodes;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nNodes; k += gridDim.x * blockDim.x) {
         const int2 l = nodeLink[k];
-        const long long word = (long long) (unsigned) l.x | ((long long) l.y << 32);
-        const double* Q = nodeQuad + 6 * (size_t) k;
         const bool body = l.y >= 0;
+        const int who = body ? l.y : nodeRange ? ~(k - nodeRange[k].x) : -1;
+        const long long word = (long long) (unsigned) l.x | ((long long) who << 32);
+        const double* Q = nodeQuad + 6 * (size_t) k;
         double4* r = rec + 3 * (size_t) k;
         r[0] = nodePM[k];
         r[1] = make_double4(nodeCrit[k], __longlong_as_double(word), body ? 0.0 : Q[0],
                             body ? 0.0 : Q[1]);
         r[2] = body ? make_double4(0.0, 0.0, 0.0, 0.0) : make_double4(Q[2], Q[3], Q[4], Q[5]);
-        if (body) continue;
-        int ch[8] = {-1, -1, -1, -1, -1, -1, -1, -1};      // k + 1, then Next() up to Next(k)
-        int c = k + 1;
-#pragma unroll
-        for (int m = 0; m < 8; ++m)
-            if (c < l.x) { ch[m] = c; c = nodeLink[c].x; }
-        kids[2 * (size_t) k] = make_int4(ch[0], ch[1], ch[2], ch[3]);
-        kids[2 * (size_t) k + 1] = make_int4(ch[4], ch[5], ch[6], ch[7]);
     }
 }
 
@@ -110,7 +104,7 @@ constexpr int TEAM_RING = 16;         // at most 7 listed before a cell's up to 
 struct NbTeam {
     double term[3][3 * 32 + 4];         // component: three terms of every lane (padded)
     int2 ring[TEAM_RING];               // listed: {node, cells complemented; bodies that take it}
-    // the cells with siblings below them still to list: {cell, the bodies of its eight children in
+    // the cells with children still to list: {cell's slot, the bodies of its eight children in
     // four bits each, next child | cover << 8 | open children << 16 | children that are bodies << 24}
     int4 frame[NB_GRID_LEVELS + 2];
 };
@@ -146,7 +140,7 @@ k_walk_fp64_team(const double4* __restrict__ rec, const int* __restrict__ kids,
     unsigned long long cVisit = 0, cBB = 0, cBC = 0, cSteps = 0;
 
     // the current cell's children, child p in lanes 4 p ..: node, the bodies that take it
-    int kid = -1, cellNode = -1;
+    int kid = -1, kidSlot = 0, cellSlot = 0;
     unsigned use = 0;
     unsigned todo = __ballot_sync(NB_FULL_MASK, valid) & TEAM_ALL;   // bodies whose tree is to come
     unsigned open = 0, leaf = 0;        // bit 4 p: some body opens child p; child p is a body
@@ -164,6 +158,7 @@ k_walk_fp64_team(const double4* __restrict__ rec, const int* __restrict__ kids,
         const double drSq = dz * dz + (dy * dy + dx * dx);
         const bool mine = kid >= 0 && !((cover >> b) & 1u);     // this body still walks here
         const bool body = kid >= 0 && bodyIndex >= 0;
+        kidSlot = ~bodyIndex;
         const bool self = mine && body && (unsigned) bodyIndex == j;
         const bool take = mine && (body ? !self : drSq >= r1.x);
         metSelf |= self;
@@ -234,8 +229,10 @@ k_walk_fp64_team(const double4* __restrict__ rec, const int* __restrict__ kids,
                 --level;
                 __syncwarp();
                 const int4 f = T.frame[level];
-                cellNode = f.x;
-                kid = __ldg(kids + 8 * (size_t) cellNode + p);
+                cellSlot = f.x;
+                kid = __ldg(kids + 8 * (size_t) cellSlot + p);
+                // the upper half of the record's link word
+                kidSlot = ~__ldg(reinterpret_cast<const int*>(rec + 3 * (size_t) max(kid, 0) + 1) + 3);
                 use = ((unsigned) f.y >> (4 * p)) & TEAM_ALL;
                 pos = f.z & 255;
                 cover = ((unsigned) f.z >> 8) & 255u;
@@ -264,18 +261,18 @@ k_walk_fp64_team(const double4* __restrict__ rec, const int* __restrict__ kids,
         head += __popc(adds);
         pos = stop + 1;
         if (om) {                                   // walk into it
-            const int c = __shfl_sync(NB_FULL_MASK, kid, TEAM_BODIES * stop);
+            const int c = __shfl_sync(NB_FULL_MASK, kidSlot, TEAM_BODIES * stop);
             const unsigned u = __shfl_sync(NB_FULL_MASK, use, TEAM_BODIES * stop);
             const int next = __ldg(kids + 8 * (size_t) c + p);
             if (pos < TEAM_LANES && ((taken | open) >> (TEAM_BODIES * pos)) != 0u) {
                 const unsigned uses = __reduce_or_sync(NB_FULL_MASK, use << (4 * p));
                 if (lane == 0)
-                    T.frame[level] = make_int4(cellNode, (int) uses, pos | (int) (cover << 8),
+                    T.frame[level] = make_int4(cellSlot, (int) uses, pos | (int) (cover << 8),
                                                (int) (open | leaf << 1));
                 ++level;
             }
             cover |= u;
-            cellNode = c;
+            cellSlot = c;
             kid = next;
             test();
         }
@@ -652,36 +649,31 @@ void nb_launch_body_epilogue(const double* px, const double* py, const double* p
                              const NbWalkParams& wp, const NbPot& pot, const NbScalars* sc,
                              int numSMs, cudaStream_t s, const NbForest* forest);
 
-void nb_launch_pack_walk(const double4* nodePM, const double* nodeCrit, const int2* nodeLink,
-                         const double* nodeQuad, double4* rec, int4* kids, int capNodes,
-                         const NbScalars* sc, cudaStream_t s)
+void nb_launch_pack_walk(const NbTreeBuffers& b, int capNodes, bool slots, cudaStream_t s)
 {
-    k_pack_walk<<<min((capNodes + 255) / 256, 4096), 256, 0, s>>>(nodePM, nodeCrit, nodeLink,
-                                                                  nodeQuad, rec, kids, sc);
+    k_pack_walk<<<min((capNodes + 255) / 256, 4096), 256, 0, s>>>(
+        b.nodePM, b.nodeCrit, b.nodeLink, slots ? b.nodeRange : nullptr, b.nodeQuad, b.walkRec, b.sc);
     nb_count_launch();
 }
 
 // The team walk below its line (form 0 is the per-lane walk above it).
 bool nb_walk_team(int n) { return n <= TEAM_MAX_BODIES; }
 
-void nb_launch_walk_fp64(const double4* nodePM, const double* nodeCrit, const int2* nodeLink,
-                         const double* nodeQuad, const unsigned* order, const double* px,
-                         const double* py, const double* pz, double* ax, double* ay, double* az,
-                         double* vx, double* vy, double* vz, const NbWalkParams& wp,
-                         const NbPot& pot, NbScalars* sc, bool count, cudaStream_t s,
-                         double4* walkRec, int4* walkKids, int capNodes, const NbForest* forest,
+void nb_launch_walk_fp64(const NbTreeBuffers& b, int capNodes, const NbWalkParams& wp,
+                         const NbPot& pot, bool count, cudaStream_t s, const NbForest* forest,
                          int form)
 {
     const int warps = (wp.n + 31) / 32;
     const int blocks = (warps * 32 + WALK_THREADS - 1) / WALK_THREADS;
     if (blocks <= 0) return;
-    nb_launch_pack_walk(nodePM, nodeCrit, nodeLink, nodeQuad, walkRec, walkKids, capNodes, sc, s);
+    nb_launch_pack_walk(b, capNodes, true, s);
     const NbForest f = forest ? *forest : NbForest{nullptr, nullptr, 0};
     const bool team = form == 0 && nb_walk_team(wp.n);
     const int perTeamBlock = TEAM_BODIES * WALK_THREADS / 32;
     const int teamBlocks = (wp.n + perTeamBlock - 1) / perTeamBlock;
-#define NB_LANES_ARGS walkRec, order, px, py, pz, ax, ay, az, wp, sc, f
-#define NB_TEAM_ARGS walkRec, (const int*) walkKids, order, px, py, pz, ax, ay, az, wp, sc, f
+#define NB_LANES_ARGS b.walkRec, b.sort.idxA, b.px, b.py, b.pz, b.ax, b.ay, b.az, wp, b.sc, f
+#define NB_TEAM_ARGS                                                                          \
+    b.walkRec, (const int*) b.walkKids, b.sort.idxA, b.px, b.py, b.pz, b.ax, b.ay, b.az, wp, b.sc, f
 #define NB_TEAM(FOREST)                                                                       \
     do {                                                                                      \
         if (count) k_walk_fp64_team<true, FOREST><<<teamBlocks, WALK_THREADS, 0, s>>>(NB_TEAM_ARGS); \
@@ -712,7 +704,8 @@ void nb_launch_walk_fp64(const double4* nodePM, const double* nodeCrit, const in
 #undef NB_LANES_ARGS
 #undef NB_TEAM_ARGS
     nb_count_launch();
-    nb_launch_body_epilogue(px, py, pz, ax, ay, az, vx, vy, vz, wp, pot, sc, 0, s, forest);
+    nb_launch_body_epilogue(b.px, b.py, b.pz, b.ax, b.ay, b.az, b.vx, b.vy, b.vz, wp, pot, b.sc, 0, s,
+                            forest);
 }
 
 void nb_launch_direct_fp64(const double* px, const double* py, const double* pz,
