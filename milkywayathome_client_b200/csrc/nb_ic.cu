@@ -1,4 +1,4 @@
-// Two-component dwarf initial conditions on the GPU, one thread per body.
+// Two-component dwarf initial conditions on the GPU, one warp per body.
 //
 // Restates the sampler of nbGenerateMixedDwarfCore (nbody/src/nbody_mixeddwarf.c:765-1026)
 // for the reference's dwarf profiles (Dwarf.plummer, nfw, general_hernquist and cored,
@@ -20,9 +20,10 @@
 // counter-based stream (splitmix64 of the seed and the body index), so the samples agree with
 // the reference's in distribution, not body for body.  The per-body work (tens of DF
 // evaluations of ~330 integrand points each) is what makes the reference's sampler take ~12 min
-// per 10^6 bodies on one core; here the bodies are independent threads.
+// per 10^6 bodies on one core; here the bodies are independent warps.
 #include "nb_common.cuh"
 #include "nb_crmath.cuh"
+#include "nb_rdiv.cuh"
 #include <vector>
 
 namespace {
@@ -112,24 +113,76 @@ struct NbRng {
 };
 
 // The two components of the body's dwarf as the DF evaluation sees them: potL/potD/psi/den
-// and the masses and scale lengths.  Two forms: both components Plummer, held in four
+// and the masses and scale lengths.  Two forms: both components Plummer, held in
 // registers (the common case; the potential is evaluated ~10^5 times per body), and any
 // profiles, read from the device table.
 struct NbIcPlummerModel {
     double ML, aL, MD, aD;
+    // of the body's own component: the density's constant, the scale length and its reciprocal
+    double rho, a, ra;
+    bool shared;                // masses and scales in the ranges of the shared reciprocals
+    __device__ NbIcPlummerModel(double ML_, double aL_, double MD_, double aD_, bool dark)
+        : ML(ML_), aL(aL_), MD(MD_), aD(aD_)
+    {
+        const double M = dark ? MD : ML;
+        a = dark ? aD : aL;
+        ra = 1.0 / a;
+        rho = (3.0 / (4.0 * M_PI)) * (M / (a * a * a));
+        shared = nb_exp_in<-700, 700>(ML) && nb_exp_in<-700, 700>(MD) &&
+                 nb_pos_exp_in<-49, 49>(aL) && nb_pos_exp_in<-49, 49>(aD) && !nb_near_ones(a);
+    }
     __device__ double potL(double r) const { return ML / sqrt(r * r + aL * aL); }
     __device__ double potD(double r) const { return MD / sqrt(r * r + aD * aD); }
     __device__ double psi(double r) const { return potL(r) + potD(r); }
-    __device__ double den(bool dark, double r) const
+    __device__ double den(bool, double r) const
     {
-        const double M = dark ? MD : ML, a = dark ? aD : aL;
         const double x = 1.0 + (r / a) * (r / a);
-        return (3.0 / (4.0 * M_PI)) * (M / (a * a * a)) * (1.0 / sqrt(x * x * x * x * x));
+        return rho * (1.0 / sqrt(x * x * x * x * x));
     }
     __device__ double massL() const { return ML; }
     __device__ double massD() const { return MD; }
     __device__ double scaleL() const { return aL; }
     __device__ double scaleD() const { return aD; }
+    // M / sqrt(s) with a shared reciprocal (nb_rdiv.cuh); ok falls outside its range
+    __device__ __forceinline__ static double over_root(double M, double s, bool& ok)
+    {
+        double y;
+        const double root = nb_sqrt_recip(s, nb_rsqrt_estimate(s), y);
+        ok &= nb_pos_exp_in<-100, 100>(s) && !nb_near_ones(s);
+        return nb_quot(M, root, y);
+    }
+    // potL, potD and den at the five stencil points of x, rounded as the functions above: the
+    // divisions and roots share their reciprocals, and no branch keeps the fifteen chains from
+    // overlapping
+    __device__ __forceinline__ void stencils(bool dark, double x, double (&L)[5], double (&D)[5],
+                                             double (&R)[5]) const
+    {
+        const double h = 0.001;
+        const double r[5] = {x - 2.0 * h, x - h, x, x + h, x + 2.0 * h};
+        bool ok = shared;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            L[k] = over_root(ML, r[k] * r[k] + aL * aL, ok);
+            D[k] = over_root(MD, r[k] * r[k] + aD * aD, ok);
+            const double q = nb_quot(r[k], a, ra);
+            const double w = 1.0 + q * q;
+            const double w5 = w * w * w * w * w;
+            double y;
+            const double root = nb_sqrt_recip(w5, nb_rsqrt_estimate(w5), y);
+            ok &= nb_pos_exp_in<-1, 400>(w5) && !nb_near_ones(w5);
+            R[k] = rho * nb_recip_step(root, y);
+        }
+        if (!ok) {
+#pragma unroll 1
+            for (int k = 0; k < 5; ++k) {
+                const double rk = k == 0 ? r[0] : k == 1 ? r[1] : k == 2 ? r[2] : k == 3 ? r[3] : r[4];
+                const double l = potL(rk), d = potD(rk), e = den(dark, rk);
+#pragma unroll
+                for (int q = 0; q < 5; ++q)
+                    if (q == k) { L[q] = l; D[q] = d; R[q] = e; }
+            }
+        }
+    }
 };
 struct NbIcModel {
     const NbIcComp* __restrict__ L;
@@ -142,48 +195,71 @@ struct NbIcModel {
     __device__ double massD() const { return D->M; }
     __device__ double scaleL() const { return L->a; }
     __device__ double scaleD() const { return D->a; }
+    __device__ __forceinline__ void stencils(bool dark, double x, double (&vL)[5], double (&vD)[5],
+                                             double (&vR)[5]) const
+    {
+        const double h = 0.001;
+        const double r[5] = {x - 2.0 * h, x - h, x, x + h, x + 2.0 * h};
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            vL[k] = potL(r[k]);
+            vD[k] = potD(r[k]);
+            vR[k] = den(dark, r[k]);
+        }
+    }
 };
 
-// five-point stencils with h = 0.001 (first_derivative / second_derivative)
-template <typename F>
-__device__ __forceinline__ double d1(F f, double x)
+// The five-point stencils take their values at x - 2h, x - h, x, x + h, x + 2h (h = 0.001).
+// first_derivative / second_derivative from those values
+__device__ __forceinline__ double ic_d1(const double (&v)[5])
 {
     const double h = 0.001;
-    const double p1 = 1.0 * f(x - 2.0 * h), p2 = -8.0 * f(x - h);
-    const double p3 = -1.0 * f(x + 2.0 * h), p4 = 8.0 * f(x + h);
+    const double p1 = 1.0 * v[0], p2 = -8.0 * v[1], p3 = -1.0 * v[4], p4 = 8.0 * v[3];
     return (p1 + p2 + p3 + p4) * (1.0 / (12.0 * h));
 }
-template <typename F>
-__device__ __forceinline__ double d2(F f, double x)
+__device__ __forceinline__ double ic_d2(const double (&v)[5])
 {
     const double h = 0.001;
-    const double p1 = -1.0 * f(x + 2.0 * h), p2 = 16.0 * f(x + h), p3 = -30.0 * f(x);
-    const double p4 = 16.0 * f(x - h), p5 = -1.0 * f(x - 2.0 * h);
+    const double p1 = -1.0 * v[4], p2 = 16.0 * v[3], p3 = -30.0 * v[2];
+    const double p4 = 16.0 * v[1], p5 = -1.0 * v[0];
     return (p1 + p2 + p3 + p4 + p5) * (1.0 / (12.0 * h * h));
 }
 
 // the DF integrand d^2 rho / d psi^2 / sqrt(|E - psi|) at radius ri (fun)
 template <typename Model>
-__device__ double ic_integrand(const Model& m, double ri, double energy, bool dark)
+__device__ __forceinline__ double ic_integrand(const Model& m, double ri, double energy, bool dark)
 {
-    auto potL = [&](double r) { return m.potL(r); };
-    auto potD = [&](double r) { return m.potD(r); };
-    auto denC = [&](double r) { return m.den(dark, r); };
-    double dpsi = d1(potL, ri) + d1(potD, ri);
-    const double d2psi = d2(potL, ri) + d2(potD, ri);
-    const double dden = d1(denC, ri), d2den = d2(denC, ri);
+    double L[5], D[5], R[5];
+    m.stencils(dark, ri, L, D, R);
+    double dpsi = ic_d1(L) + ic_d1(D);
+    const double d2psi = ic_d2(L) + ic_d2(D);
+    const double dden = ic_d1(R), d2den = ic_d2(R);
     if (dpsi == 0.0) dpsi = 1.0e-6;
     const double dsq = d2den * (1.0 / dpsi) - dden * d2psi * (1.0 / (dpsi * dpsi));
-    const double diff = fabs(energy - m.psi(ri));
+    const double diff = fabs(energy - (L[2] + D[2]));
     const double denom = diff != 0.0 ? 1.0 / sqrt(diff)
                                      : 1.0 / sqrt(fabs(energy - m.psi(ri + 0.0001)));
     return dsq * denom;
 }
 
+// A warp samples one body.  Its lanes follow the body's rejections and searches together and
+// share out what a step evaluates many of: the quadrature's 330 integrand points (ten panels of
+// three points at a time) and the bisection's midpoints (the 31 of its next five steps).  Sums
+// and decisions keep the order of the one-thread form, so the samples are the same bit for bit.
+// A body takes 10 to 60 evaluations of the distribution function of 330 x ~450 FP64 operations
+// each: with a thread a body the warps waited for their longest body and a few long ones set
+// the time (eight dwarfs of 4,096 to 65,536 bodies: 185 -> 83 ms, and 62 with the shared
+// reciprocals of NbIcPlummerModel::stencils).  FP64 issue and its dependences bound it now; five
+// resident blocks (96 registers, a few spilled) beat four by 2 % and three by 10 %.
+struct NbIcWarp {
+    int lane;
+    double* terms;              // 32 doubles of shared memory
+};
+
 // composite three-point Gauss quadrature: 100 panels over [a, 1.5 a], then 10 up to b
 template <typename Model>
-__device__ double ic_gauss_quad(const Model& m, double lower, double upper, double energy,
-                                bool dark)
+__device__ double ic_gauss_quad(const NbIcWarp& w, const Model& m, double lower, double upper,
+                                double energy, bool dark)
 {
     const double a = lower > upper ? upper : lower, b = lower > upper ? lower : upper;
     const double benchmark = 1.5 * a;
@@ -192,45 +268,70 @@ __device__ double ic_gauss_quad(const Model& m, double lower, double upper, doub
     double coef2 = (lowerg + upperg) / 2.0, coef1 = (upperg - lowerg) / 2.0;
     const double c1 = 0.55555555555, c2 = 0.88888888888, c3 = 0.55555555555;
     const double x1 = -0.77459666924, x3 = 0.77459666924;
+    const int panel = w.lane / 3, point = w.lane % 3;       // of the ten panels at a time
     double intv = 0.0;
-    for (int counter = 0; counter <= 100000; ++counter) {
-        const double x1n = coef1 * x1 + coef2, x2n = coef2, x3n = coef1 * x3 + coef2;
-        intv = intv + c1 * ic_integrand(m, x1n, energy, dark) * coef1 +
-               c2 * ic_integrand(m, x2n, energy, dark) * coef1 +
-               c3 * ic_integrand(m, x3n, energy, dark) * coef1;
-        lowerg = upperg;
-        upperg = upperg + hg;
-        coef2 = (lowerg + upperg) / 2.0;
-        coef1 = (upperg - lowerg) / 2.0;
-        if (lowerg > benchmark) hg = (b - benchmark) / 10.0;
-        if (upper > lower) { if (lowerg >= upper) break; }
-        else if (lower > upper) { if (lowerg >= lower) break; }
+    int counter = 0;
+    for (bool done = false; !done;) {
+        double my1 = 0.0, my2 = 0.0;
+        int panels = 0;
+        for (; panels < 10 && !done; ++panels) {
+            if (panel == panels) { my1 = coef1; my2 = coef2; }
+            lowerg = upperg;
+            upperg = upperg + hg;
+            coef2 = (lowerg + upperg) / 2.0;
+            coef1 = (upperg - lowerg) / 2.0;
+            if (lowerg > benchmark) hg = (b - benchmark) / 10.0;
+            if (upper > lower) { if (lowerg >= upper) done = true; }
+            else if (lower > upper) { if (lowerg >= lower) done = true; }
+            if (++counter > 100000) done = true;
+        }
+        double term = 0.0;
+        if (panel < panels) {
+            const double x = point == 0 ? my1 * x1 + my2 : point == 1 ? my2 : my1 * x3 + my2;
+            const double c = point == 0 ? c1 : point == 1 ? c2 : c3;
+            term = c * ic_integrand(m, x, energy, dark) * my1;
+        }
+        __syncwarp();
+        w.terms[w.lane] = term;
+        __syncwarp();
+        for (int t = 0; t < 3 * panels; ++t) intv = intv + w.terms[t];
     }
     return lower > upper ? -intv : intv;
 }
 
 // bisection for psi(r) = value on [lo, hi] split in 4 intervals (root_finder); 0 if none
 template <typename Model>
-__device__ double ic_root(const Model& m, double value, double lo, double hi)
+__device__ double ic_root(const NbIcWarp& w, const Model& m, double value, double lo, double hi)
 {
-    double vals[5], bounds[5];
-    for (int i = 0; i < 5; ++i) {
-        double x = ((hi - lo) * (double) i) / 4.0 + lo;
-        double v = m.psi(x) - value;
-        if (isnan(v)) { x += 0.0001; v = m.psi(x) - value; }
-        vals[i] = v;
-        bounds[i] = x;
-    }
+    double x = ((hi - lo) * (double) min(w.lane, 4)) / 4.0 + lo;
+    double v = m.psi(x) - value;
+    if (isnan(v)) { x += 0.0001; v = m.psi(x) - value; }
     for (int q = 0; q < 4; ++q) {
+        const double v0 = __shfl_sync(NB_FULL_MASK, v, q), v1 = __shfl_sync(NB_FULL_MASK, v, q + 1);
+        const double b0 = __shfl_sync(NB_FULL_MASK, x, q), b1 = __shfl_sync(NB_FULL_MASK, x, q + 1);
         double nlo, nhi;
-        if (vals[q] < 0 && vals[q + 1] > 0) { nlo = bounds[q]; nhi = bounds[q + 1]; }
-        else if (vals[q] > 0 && vals[q + 1] < 0) { nlo = bounds[q + 1]; nhi = bounds[q]; }
+        if (v0 < 0 && v1 > 0) { nlo = b0; nhi = b1; }
+        else if (v0 > 0 && v1 < 0) { nlo = b1; nhi = b0; }
         else continue;
         double mid = 0.0, f = 1.0;
-        for (int counter = 0; fabs(f) > .0001 && counter <= 10000; ++counter) {
-            mid = (nlo + nhi) / 2.0;
-            f = m.psi(mid) - value;
-            if (f < 0.0) nlo = mid; else nhi = mid;
+        int counter = 0;
+        while (fabs(f) > .0001 && counter <= 10000) {
+            // lane h (1 .. 31) holds the midpoint reached from here by the steps that the bits of
+            // h after its first one spell: a one where psi - value was negative
+            double l = nlo, r = nhi;
+            const int h0 = max(w.lane, 1);
+            for (int d = 30 - __clz(h0); d >= 0; --d) {
+                const double c = (l + r) / 2.0;
+                if ((h0 >> d) & 1) l = c; else r = c;
+            }
+            const double myMid = (l + r) / 2.0;
+            const double myF = m.psi(myMid) - value;
+            for (int h = 1; h < 32 && fabs(f) > .0001 && counter <= 10000; ++counter) {
+                mid = __shfl_sync(NB_FULL_MASK, myMid, h);
+                f = __shfl_sync(NB_FULL_MASK, myF, h);
+                if (f < 0.0) { nlo = mid; h = 2 * h + 1; }
+                else { nhi = mid; h = 2 * h; }
+            }
         }
         return mid;
     }
@@ -239,7 +340,7 @@ __device__ double ic_root(const Model& m, double value, double lo, double hi)
 
 // the Eddington DF at speed v and radius r (dist_fun)
 template <typename Model>
-__device__ double ic_df(const Model& m, double v, double r, bool dark)
+__device__ double ic_df(const NbIcWarp& w, const Model& m, double v, double r, bool dark)
 {
     const double cons = 0.03582244801567226;
     const double energy = m.psi(r) - 0.5 * v * v;
@@ -250,34 +351,36 @@ __device__ double ic_df(const Model& m, double v, double r, bool dark)
         range = 100.0 * range;
         if (counter > 100) { range = 100.0 * (aL + aD); break; }
     }
-    double up = ic_root(m, energy, 0.0, range);
+    double up = ic_root(w, m, energy, 0.0, range);
     if (isinf(up) || up == 0.0 || isnan(up)) up = r;        // find_upperlimit_r's fallback
     up = fabs(up);
     const double lo = 10.0 * up;
-    return v * v * cons * ic_gauss_quad(m, lo, up, energy, dark);
+    return v * v * cons * ic_gauss_quad(w, m, lo, up, energy, dark);
 }
 
 // golden-section search for the DF maximum over speeds (max_finder)
 template <typename Model>
-__device__ double ic_df_max(const Model& m, double r, bool dark, double a, double b,
-                            double c, int limit, double tol)
+__device__ double ic_df_max(const NbIcWarp& w, const Model& m, double r, bool dark, double a,
+                            double b, double c, int limit, double tol)
 {
     const double R = 0.61803399, C = 1.0 - R;
     double x0 = a, x3 = c, x1, x2;
     if (fabs(b - c) > fabs(b - a)) { x1 = b; x2 = b + (C * (c - b)); }
     else { x2 = b; x1 = b - (C * (b - a)); }
-    double f1 = -ic_df(m, x1, r, dark), f2 = -ic_df(m, x2, r, dark);
-    int counter = 0;
-    while (fabs(x3 - x0) > (tol * (fabs(x1) + fabs(x2)))) {
-        ++counter;
-        if (f2 < f1) {
-            x0 = x1; x1 = x2; x2 = R * x2 + C * x3;
-            f1 = f2; f2 = -ic_df(m, x2, r, dark);
-        } else {
-            x3 = x2; x2 = x1; x1 = R * x1 + C * x0;
-            f2 = f1; f1 = -ic_df(m, x1, r, dark);
-        }
-        if (counter > limit) break;
+    double f1 = 0.0, f2 = 0.0;
+    // one call of ic_df in the code (its quadrature is inlined): first at x1, then x2, then the
+    // point each step replaces
+    int counter = -2;
+    bool second = false;
+    for (;;) {
+        const double f = -ic_df(w, m, second ? x2 : x1, r, dark);
+        if (second) f2 = f; else f1 = f;
+        if (++counter == -1) { second = true; continue; }
+        if (counter > limit) break;                 // counter: the steps taken
+        if (!(fabs(x3 - x0) > (tol * (fabs(x1) + fabs(x2))))) break;
+        second = f2 < f1;
+        if (second) { x0 = x1; x1 = x2; x2 = R * x2 + C * x3; f1 = f2; }
+        else { x3 = x2; x2 = x1; x1 = R * x1 + C * x0; f2 = f1; }
     }
     return f1 < f2 ? -f1 : -f2;
 }
@@ -315,7 +418,7 @@ __device__ int ic_dwarf_of(const NbIcDwarf* dw, int nD, int i)
 
 // The radius and speed of one body by rejection (r_mag, vel_mag); r = v = 0 when either fails.
 template <typename Model>
-__device__ void ic_sample_rv(const Model& m, const NbIcComp& comp, bool dark, NbRng& rng,
+__device__ void ic_sample_rv(const NbIcWarp& w, const Model& m, const NbIcComp& comp, bool dark, NbRng& rng,
                              double& rOut, double& vOut)
 {
     double r = 0.0;
@@ -330,13 +433,13 @@ __device__ void ic_sample_rv(const Model& m, const NbIcComp& comp, bool dark, Nb
     double v = 0.0;
     if (isfinite(r) && r != 0.0) {
         const double vesc = 0.99 * sqrt(fabs(2.0 * m.psi(r)));
-        const double dfMax = ic_df_max(m, r, dark, 0.0, 0.5 * vesc, vesc, 10, 1.0e-2);
+        const double dfMax = ic_df_max(w, m, r, dark, 0.0, 0.5 * vesc, vesc, 10, 1.0e-2);
         for (int tries = 0; tries <= 1000 && !(isfinite(v) && v != 0.0); ++tries) {
             v = 0.0;
             for (int counter = 0; counter <= 1000; ++counter) {  // vel_mag
                 const double vv = rng.uniform() * vesc;
                 const double u = rng.uniform();
-                if (fabs(ic_df(m, vv, r, dark) / dfMax) > u) { v = vv; break; }
+                if (fabs(ic_df(w, m, vv, r, dark) / dfMax) > u) { v = vv; break; }
             }
         }
     }
@@ -344,17 +447,21 @@ __device__ void ic_sample_rv(const Model& m, const NbIcComp& comp, bool dark, Nb
     vOut = v;
 }
 
-// One body per thread: radius and speed by rejection, isotropic directions.  ALL_PLUMMER: every
+// One body per warp: radius and speed by rejection, isotropic directions.  ALL_PLUMMER: every
 // dwarf of the table has two Plummer components (their model in registers).
+constexpr int kIcWarps = 4;
 template <bool ALL_PLUMMER>
-__global__ void k_ic_sample(const NbIcDwarf* __restrict__ dwarfs, int nD, int n,
+__global__ void __launch_bounds__(32 * kIcWarps, 5)
+k_ic_sample(const NbIcDwarf* __restrict__ dwarfs, int nD, int n,
                             double* __restrict__ px, double* __restrict__ py,
                             double* __restrict__ pz, double* __restrict__ vx,
                             double* __restrict__ vy, double* __restrict__ vz,
                             double* __restrict__ mass, int* __restrict__ types,
                             NbScalars* __restrict__ sc)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    __shared__ double terms[kIcWarps][32];
+    const NbIcWarp w{(int) (threadIdx.x & 31), terms[threadIdx.x >> 5]};
+    for (int i = blockIdx.x * kIcWarps + (threadIdx.x >> 5); i < n; i += gridDim.x * kIcWarps) {
         const NbIcDwarf& d = dwarfs[ic_dwarf_of(dwarfs, nD, i)];
         const int k = i - d.first;
         const bool dark = k >= d.nBaryon;
@@ -362,11 +469,11 @@ __global__ void k_ic_sample(const NbIcDwarf* __restrict__ dwarfs, int nD, int n,
         const NbIcComp& comp = dark ? d.D : d.L;
         double r, v;
         if (ALL_PLUMMER) {
-            const NbIcPlummerModel m{d.L.M, d.L.a, d.D.M, d.D.a};
-            ic_sample_rv(m, comp, dark, rng, r, v);
+            const NbIcPlummerModel m(d.L.M, d.L.a, d.D.M, d.D.a, dark);
+            ic_sample_rv(w, m, comp, dark, rng, r, v);
         } else {
             const NbIcModel m{&d.L, &d.D};
-            ic_sample_rv(m, comp, dark, rng, r, v);
+            ic_sample_rv(w, m, comp, dark, rng, r, v);
         }
         if (!(isfinite(r) && r != 0.0 && isfinite(v) && v != 0.0)) {
             nb_raise(sc, NBODY_ERROR);                // the reference exits here
@@ -375,6 +482,7 @@ __global__ void k_ic_sample(const NbIcDwarf* __restrict__ dwarfs, int nD, int n,
         double dv[3], dr[3];
         ic_direction(rng, v, dv);
         ic_direction(rng, r, dr);
+        if (w.lane != 0) continue;
         px[i] = dr[0]; py[i] = dr[1]; pz[i] = dr[2];
         vx[i] = dv[0]; vy[i] = dv[1]; vz[i] = dv[2];
         const int nDark = d.count - d.nBaryon;
@@ -543,15 +651,15 @@ int nb_launch_ic(const NBodyCudaMixedDwarf* host, int nD, const int* firsts, voi
     cudaMemcpyAsync(dTable, t.data(), sizeof(NbIcDwarf) * nD, cudaMemcpyHostToDevice, s);
     cudaMemsetAsync(scratch, 0, sizeof(double) * 12 * (size_t) nD, s);
     const NbIcDwarf* dt = (const NbIcDwarf*) dTable;
-    // few bodies per thread, many threads: the per-body work is long and uneven
-    const int g = min((n + 127) / 128, numSMs * 64);
+    // few bodies per warp, many warps: the per-body work is long and uneven
+    const int g = min((n + kIcWarps - 1) / kIcWarps, numSMs * 64);
     bool allPlummer = true;
     for (const NbIcDwarf& d : t)
         allPlummer = allPlummer && d.L.type == NBCUDA_DWARF_PLUMMER && d.D.type == NBCUDA_DWARF_PLUMMER;
     if (allPlummer)
-        k_ic_sample<true><<<g, 128, 0, s>>>(dt, nD, n, b.px, b.py, b.pz, b.vx, b.vy, b.vz, b.mass, types, sc);
+        k_ic_sample<true><<<g, 32 * kIcWarps, 0, s>>>(dt, nD, n, b.px, b.py, b.pz, b.vx, b.vy, b.vz, b.mass, types, sc);
     else
-        k_ic_sample<false><<<g, 128, 0, s>>>(dt, nD, n, b.px, b.py, b.pz, b.vx, b.vy, b.vz, b.mass, types, sc);
+        k_ic_sample<false><<<g, 32 * kIcWarps, 0, s>>>(dt, nD, n, b.px, b.py, b.pz, b.vx, b.vy, b.vz, b.mass, types, sc);
     const int g2 = min((n + 255) / 256, numSMs * 8);
     k_ic_moments<<<2 * nD, kIcMomentThreads, 0, s>>>(dt, nD, b.px, b.py, b.pz, b.vx, b.vy, b.vz,
                                                      b.mass, scratch);

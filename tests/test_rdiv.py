@@ -31,6 +31,17 @@ extern "C" void radial(const double* s, const double* m, const double* a, int n,
         out[5 * i + 4] = nb_quot(a[i], s[i], z);
     }
 }
+extern "C" void plummer(const double* s, const double* m, const double* x, const double* a, int n,
+                        double* out)
+{
+    for (int i = 0; i < n; ++i) {
+        double y;
+        const double r = nb_sqrt_recip(s[i], nb_rsqrt_estimate(s[i]), y);
+        out[3 * i] = nb_quot(m[i], r, y);                   // m / sqrt(s)
+        out[3 * i + 1] = nb_recip_step(r, y);               // 1 / sqrt(s)
+        out[3 * i + 2] = nb_quot(x[i], a[i], 1.0 / a[i]);   // x / a
+    }
+}
 extern "C" void ranges(const double* x, int n, int* out)
 {
     for (int i = 0; i < n; ++i)
@@ -110,6 +121,24 @@ def test_operands_next_to_rounding_boundaries(lib):
                      np.nextafter(0.25, 0), np.nextafter(0.5, 1)])
     g = np.array(np.meshgrid(edge, edge, edge)).reshape(3, -1)
     _check(lib, *g)
+
+
+@pytest.mark.parametrize("hi", [100, 400])
+def test_plummer_terms(lib, hi):
+    """The dwarf sampler's M / sqrt(r^2 + a^2), 1 / sqrt(x^5) (x^5 up to 2^400) and r / a."""
+    rng = np.random.default_rng(hi)
+    n = 500_000
+    s = _random(rng, n, -100 if hi == 100 else 0, hi)
+    m, x, a = _random(rng, n, -20, 20), _random(rng, n, -60, 45), _random(rng, n, -49, 49)
+    x[:100] = 0.0
+    x *= rng.choice([-1.0, 1.0], n)
+    out = np.empty((n, 3))
+    lib.plummer(*[v.ctypes.data_as(ctypes.c_void_p) for v in (s, m, x, a)], ctypes.c_int(n),
+                out.ctypes.data_as(ctypes.c_void_p))
+    want = np.stack([m / np.sqrt(s), 1.0 / np.sqrt(s), np.abs(x / a)], 1)
+    out[:, 2] = np.abs(out[:, 2])           # the sign of a zero quotient is not kept
+    ok = ~_near_ones(s)[:, None] & ~np.stack([np.zeros(n, bool)] * 2 + [_near_ones(a)], 1)
+    assert np.array_equal(out.view(np.uint64)[ok], want.view(np.uint64)[ok])
 
 
 def test_ranges(lib):
