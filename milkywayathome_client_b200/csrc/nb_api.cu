@@ -30,7 +30,7 @@ void nb_launch_step_adjoint(NbTreeBuffers& b, double* nodeBar, int capNodes, int
 void nb_launch_direct_fp64(const double* px, const double* py, const double* pz,
                            const double* mass, double* ax, double* ay, double* az, double* vx,
                            double* vy, double* vz, const NbWalkParams& wp, const NbPot& pot,
-                           NbScalars* sc, cudaStream_t s);
+                           NbScalars* sc, int numSMs, cudaStream_t s);
 void nb_launch_ext_only(const double* dpos, double* dacc, int n, const NbPot& pot, cudaStream_t s);
 int nb_launch_ic(const NBodyCudaMixedDwarf* host, int nD, const int* firsts, void* dTable,
                  double* scratch, NbTreeBuffers& b, int* types, int n, int numSMs, NbScalars* sc,
@@ -498,7 +498,7 @@ static NBodyCudaStatus nb_force(const NBodyCudaCtx* ctx, NBodyCudaState* st, int
             }
             rec(st->ev0);
             nb_launch_direct_fp64(b.px, b.py, b.pz, b.mass, b.ax, b.ay, b.az, b.vx, b.vy, b.vz, wp,
-                                  pot, b.sc, s);
+                                  pot, b.sc, st->numSMs, s);
             rec(st->ev1);
         } else {
             nb_build_tree(b, n, ctx->criterion, ctx->theta, ctx->useQuad, drift, ctx->timestep,

@@ -51,9 +51,10 @@ __global__ void k_pack_walk(const double4* __restrict__ nodePM, const double* __
 // and 2^700 keep every intermediate and every residual normal; the operators take the rest, and
 // the divisors next to an all-ones significand.
 // ALWAYS: the quadrupole's factors are formed whether or not this lane's node is a cell (no branch).
+// Returns whether the operands are in those ranges.
 template <bool ALWAYS>
-__device__ __forceinline__ void nb_radial(double s, double m, bool need, bool cell, double drQdr,
-                                          double& mor3, double& dr5inv, double& phiQ)
+__device__ __forceinline__ bool nb_radial_shared(double s, double m, bool cell, double drQdr,
+                                                 double& mor3, double& dr5inv, double& phiQ)
 {
     double y;
     const double drab = nb_sqrt_recip(s, nb_rsqrt_estimate(s), y);
@@ -67,14 +68,27 @@ __device__ __forceinline__ void nb_radial(double s, double m, bool need, bool ce
         phiQ = nb_quot(a, s, z);
         ok = ok && (!cell || (nb_exp_in<-700, 700>(a) && !nb_near_ones(t)));
     }
-    if (need && !ok) {
-        const double root = sqrt(s);
-        mor3 = (m / root) / s;
-        if (cell) {
-            dr5inv = 1.0 / ((s * s) * root);
-            phiQ = 2.5 * (dr5inv * drQdr) / s;
-        }
+    return ok;
+}
+
+// The operators' forms.
+__device__ __forceinline__ void nb_radial_general(double s, double m, bool cell, double drQdr,
+                                                  double& mor3, double& dr5inv, double& phiQ)
+{
+    const double root = sqrt(s);
+    mor3 = (m / root) / s;
+    if (cell) {
+        dr5inv = 1.0 / ((s * s) * root);
+        phiQ = 2.5 * (dr5inv * drQdr) / s;
     }
+}
+
+template <bool ALWAYS>
+__device__ __forceinline__ void nb_radial(double s, double m, bool need, bool cell, double drQdr,
+                                          double& mor3, double& dr5inv, double& phiQ)
+{
+    const bool ok = nb_radial_shared<ALWAYS>(s, m, cell, drQdr, mor3, dr5inv, phiQ);
+    if (need && !ok) nb_radial_general(s, m, cell, drQdr, mor3, dr5inv, phiQ);
 }
 
 // The team walk: a warp walks for TEAM_BODIES consecutive bodies, TEAM_LANES lanes each (lane =
@@ -486,42 +500,92 @@ void nb_launch_body_epilogue(const double* px, const double* py, const double* p
     nb_count_launch();
 }
 
-// nbGravity_Exact (nbody/src/nbody_grav.c:205-227): direct sum over all bodies in input
-// order (the self term contributes 0 * dr).  One thread per body; sources staged in tiles.
+// nbGravity_Exact (nbody/src/nbody_grav.c:205-227): direct sum over all bodies in input order
+// (the self term contributes 0 * dr).  H lanes share a body: each forms the terms of every H-th
+// group of EXACT_UNROLL sources, EXACT_UNROLL independent root-and-division chains at once with
+// the next group's loads behind them, and the terms are added one after another in input order
+// (lane by lane through shuffles).  Bound by the FP64 pipe, 31 operations a pair, once enough
+// warps are resident; a warp alone on its scheduler, the usual case here, waits for its own
+// chains (116 cycles a source where the pipe takes 62).  A thread a body in blocks of 256, one
+// chain at a time, took 2.24 ms at 10,007 bodies and 0.23 at 1,000; now 0.59 and 0.041.  H = 1 / 2 /
+// 4 in ms: 4,000 bodies 0.244 / 0.175 / 0.135, 7,000 0.420 / 0.304 / 0.357, 10,007 0.593 / 0.693 /
+// 0.779, 20,000 2.03 / 2.11 / 2.50 (4.46 before), 30,000 3.03 / 4.08 / 5.20.
 constexpr int EXACT_TILE = 256;
-__global__ void __launch_bounds__(EXACT_TILE)
+constexpr int EXACT_UNROLL = 8;
+template <int H>
+__global__ void __launch_bounds__(32)
 k_direct_fp64(const double* __restrict__ px, const double* __restrict__ py,
               const double* __restrict__ pz, const double* __restrict__ mass,
               double* __restrict__ ax, double* __restrict__ ay, double* __restrict__ az,
-              double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,
-              NbWalkParams wp, NbPot pot, NbScalars* __restrict__ sc)
+              NbWalkParams wp)
 {
-    __shared__ double4 tile[EXACT_TILE];
+    constexpr int U = EXACT_UNROLL;
     const int n = wp.n;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int h = lane % H;
+    const int i = blockIdx.x * (32 / H) + lane / H;
     const bool valid = i < n;
     const double x0 = valid ? px[i] : 0.0, y0 = valid ? py[i] : 0.0, z0 = valid ? pz[i] : 0.0;
     const double eps2 = wp.eps2;
-    double accx = 0.0, accy = 0.0, accz = 0.0;
-    for (int base = 0; base < n; base += EXACT_TILE) {
-        const int k = base + threadIdx.x;
-        __syncthreads();
-        tile[threadIdx.x] = k < n ? make_double4(px[k], py[k], pz[k], mass[k]) : make_double4(0, 0, 0, 0);
-        __syncthreads();
-        const int lim = min(EXACT_TILE, n - base);
-        for (int t = 0; t < lim; ++t) {
-            const double4 b = tile[t];
-            const double dx = b.x - x0, dy = b.y - y0, dz = b.z - z0;
-            const double drSq = (dz * dz + (dy * dy + dx * dx)) + eps2;
-            const double drab = sqrt(drSq);
-            const double phii = b.w / drab;
-            const double mor3 = phii / drSq;
-            accx = accx + mor3 * dx;
-            accy = accy + mor3 * dy;
-            accz = accz + mor3 * dz;
+    double acc[3] = {0.0, 0.0, 0.0};
+    double x[U], y[U], z[U], m[U];
+    auto fetch = [&](int k0) {
+        if (k0 + U <= n) {
+#pragma unroll
+            for (int u = 0; u < U; u += 4) {            // k0 is a multiple of 8: 32-byte aligned
+                const double4 a = nb_ld32(reinterpret_cast<const double4*>(px + k0 + u));
+                const double4 b = nb_ld32(reinterpret_cast<const double4*>(py + k0 + u));
+                const double4 c = nb_ld32(reinterpret_cast<const double4*>(pz + k0 + u));
+                const double4 d = nb_ld32(reinterpret_cast<const double4*>(mass + k0 + u));
+                x[u] = a.x; x[u + 1] = a.y; x[u + 2] = a.z; x[u + 3] = a.w;
+                y[u] = b.x; y[u + 1] = b.y; y[u + 2] = b.z; y[u + 3] = b.w;
+                z[u] = c.x; z[u + 1] = c.y; z[u + 2] = c.z; z[u + 3] = c.w;
+                m[u] = d.x; m[u + 1] = d.y; m[u + 2] = d.z; m[u + 3] = d.w;
+            }
+        } else {                                        // past the end: the last body, taken as none
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int k = min(k0 + u, n - 1);
+                x[u] = px[k]; y[u] = py[k]; z[u] = pz[k]; m[u] = mass[k];
+            }
         }
+    };
+    fetch(U * h);
+    for (int base = 0; base < n; base += U * H) {
+        const int k0 = base + U * h;
+        // one test for all: a branch a source would keep the chains from overlapping
+        double t[U][3], r2[U], mm[U], mor3[U], dr5inv, phiQ;
+        bool ok = true;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            t[u][0] = x[u] - x0; t[u][1] = y[u] - y0; t[u][2] = z[u] - z0;
+            r2[u] = (t[u][2] * t[u][2] + (t[u][1] * t[u][1] + t[u][0] * t[u][0])) + eps2;
+            mm[u] = m[u];
+        }
+        fetch(k0 + U * H);                              // the next sources, behind this arithmetic
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            ok &= nb_radial_shared<false>(r2[u], mm[u], false, 0.0, mor3[u], dr5inv, phiQ);
+        if (!ok)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                nb_radial_general(r2[u], mm[u], false, 0.0, mor3[u], dr5inv, phiQ);
+        // the sum never is -0, so a zero term leaves it as it is
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) t[u][c] = k0 + u < n ? mor3[u] * t[u][c] : 0.0;
+#pragma unroll
+        for (int q = 0; q < H; ++q)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    acc[c] = acc[c] + (H == 1 ? t[u][c]
+                                              : __shfl_sync(NB_FULL_MASK, t[u][c], lane - h + q));
     }
-    if (valid) nb_finish_body(pot, wp, (unsigned) i, x0, y0, z0, accx, accy, accz, ax, ay, az, vx, vy, vz);
+    // self-gravity only; k_body_epilogue adds the external potential and kicks
+    if (valid && h == 0) { ax[i] = acc[0]; ay[i] = acc[1]; az[i] = acc[2]; }
 }
 
 // Direct FP64 sums (nbGravity_Exact arithmetic) for a sample of target bodies: the accuracy
@@ -711,12 +775,19 @@ void nb_launch_walk_fp64(const NbTreeBuffers& b, int capNodes, const NbWalkParam
 void nb_launch_direct_fp64(const double* px, const double* py, const double* pz,
                            const double* mass, double* ax, double* ay, double* az, double* vx,
                            double* vy, double* vz, const NbWalkParams& wp, const NbPot& pot,
-                           NbScalars* sc, cudaStream_t s)
+                           NbScalars* sc, int numSMs, cudaStream_t s)
 {
-    const int blocks = (wp.n + EXACT_TILE - 1) / EXACT_TILE;
-    if (blocks <= 0) return;
-    k_direct_fp64<<<blocks, EXACT_TILE, 0, s>>>(px, py, pz, mass, ax, ay, az, vx, vy, vz, wp, pot, sc);
+    if (wp.n <= 0) return;
+    // the most lanes a body that leave one warp a scheduler (4 an SM): past that the warps take
+    // turns, and sharing a body only adds the shuffles
+    const int slots = 32 * 4 * numSMs;
+    const int H = 4ll * wp.n <= slots ? 4 : 2ll * wp.n <= slots ? 2 : 1;
+    const int blocks = (wp.n + 32 / H - 1) / (32 / H);
+    if (H == 4) k_direct_fp64<4><<<blocks, 32, 0, s>>>(px, py, pz, mass, ax, ay, az, wp);
+    else if (H == 2) k_direct_fp64<2><<<blocks, 32, 0, s>>>(px, py, pz, mass, ax, ay, az, wp);
+    else k_direct_fp64<1><<<blocks, 32, 0, s>>>(px, py, pz, mass, ax, ay, az, wp);
     nb_count_launch();
+    nb_launch_body_epilogue(px, py, pz, ax, ay, az, vx, vy, vz, wp, pot, sc, numSMs, s, nullptr);
 }
 
 void nb_launch_ext_only(const double* dpos, double* dacc, int n, const NbPot& pot, cudaStream_t s)

@@ -1,0 +1,35 @@
+"""The Exact criterion's direct sum at the edges of its split, on a GPU: part-filled groups of
+sources, one, two and four lanes a body (the lines lie at 4,736 and 9,472 bodies on 148 SMs), and
+operands its shared reciprocals leave to the operators; bit for bit the oracle's."""
+import numpy as np
+import pytest
+
+from conftest import bits_equal, make_ctx
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 15, 17, 31, 32, 33, 63, 65, 4735, 4736, 4737, 9472, 9473])
+def test_sizes_equal_the_oracle(n):
+    from milkywayathome_client_b200 import NBodyState, models
+    from oracle import bindings as ob
+    pos, vel, mass, _ = models.plummer_plummer_dwarf(n, seed=70 + n)
+    ctx = make_ctx(max(n, 2), criterion="Exact")
+    rc, want, _, _ = ob.grav_map(ctx.struct, pos, mass, ctx.treeRSize)
+    with NBodyState.create(ctx, pos, vel, mass, gravmap=False) as st:
+        assert st.gravMap(ctx) == rc
+        assert bits_equal(st.accels(), want)
+
+
+@pytest.mark.parametrize("eps2,scale", [(0.0, 1.0), (2.0 ** -120, 1.0), (0.01, 2.0 ** -715),
+                                        (0.01, 2.0 ** 705), (0.01, 0.0)])
+def test_operands_outside_the_shared_ranges(eps2, scale):
+    from milkywayathome_client_b200 import NBodyState, models
+    from oracle import bindings as ob
+    pos, vel, mass, _ = models.plummer_plummer_dwarf(300, seed=3)
+    ctx = make_ctx(300, criterion="Exact", eps2=eps2, potential=None)
+    mass = mass * scale
+    rc, want, _, _ = ob.grav_map(ctx.struct, pos, mass, ctx.treeRSize)
+    with NBodyState.create(ctx, pos, vel, mass, gravmap=False) as st:
+        assert st.gravMap(ctx) == rc
+        assert np.array_equal(st.accels(), want, equal_nan=True)
