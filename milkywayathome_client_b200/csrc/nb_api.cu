@@ -501,9 +501,8 @@ static NBodyCudaStatus nb_force(const NBodyCudaCtx* ctx, NBodyCudaState* st, int
                                   pot, b.sc, st->numSMs, s);
             rec(st->ev1);
         } else {
-            nb_build_tree(b, n, ctx->criterion, ctx->theta, ctx->useQuad, drift, ctx->timestep,
-                          st->numSMs, s, shift0);
-            nb_link_and_moments(b, n, st->capNodes, ctx->criterion, ctx->theta, ctx->useQuad, s);
+            nb_build_tree(b, n, st->capNodes, ctx->criterion, ctx->theta, ctx->useQuad, drift,
+                          ctx->timestep, st->numSMs, s, shift0);
             rec(st->ev0);
             if (mixed)
                 nb_launch_walk_mixed(b, st->mx, st->capNodes, wp, pot, st->counting != 0,
@@ -869,10 +868,8 @@ NBodyCudaStatus nbMakeTreeCUDA(const NBodyCudaCtx* ctx, NBodyCudaState* st)
         init.rsize = st->rsize;
         init.capNodes = st->capNodes;
         NB_CHECK(cudaMemcpyAsync(b.sc, &init, sizeof init, cudaMemcpyHostToDevice, st->stream));
-        nb_build_tree(b, st->nbody, ctx->criterion, ctx->theta, ctx->useQuad, 0, 0.0, st->numSMs,
-                      st->stream);
-        nb_link_and_moments(b, st->nbody, st->capNodes, ctx->criterion, ctx->theta, ctx->useQuad,
-                            st->stream);
+        nb_build_tree(b, st->nbody, st->capNodes, ctx->criterion, ctx->theta, ctx->useQuad, 0, 0.0,
+                      st->numSMs, st->stream);
         NB_CHECK(cudaGetLastError());
         NB_CHECK(cudaMemcpyAsync(st->scHost, b.sc, sizeof(NbScalars), cudaMemcpyDeviceToHost,
                                  st->stream));

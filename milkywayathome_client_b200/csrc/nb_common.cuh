@@ -322,10 +322,12 @@ void nb_launch_walk_mixed(const NbTreeBuffers& b, const NbMixedBuffers& m, int c
                           const NbWalkParams& wp, const NbPot& pot, bool count, int numSMs,
                           cudaStream_t s, const NbForest* forest = nullptr);
 
-void nb_build_tree(NbTreeBuffers& b, int n, int criterion, double theta, int useQuad, int drift,
-                   double dt, int numSMs, cudaStream_t s, const double* shift = nullptr);
-void nb_link_and_moments(NbTreeBuffers& b, int n, int capNodes, int criterion, double theta,
-                         int useQuad, cudaStream_t s);
+void nb_build_tree(NbTreeBuffers& b, int n, int capNodes, int criterion, double theta, int useQuad,
+                   int drift, double dt, int numSMs, cudaStream_t s, const double* shift = nullptr);
+// The one-launch build of small systems (nb_build.cu): all of nb_build_tree but the moments.
+bool nb_build_in_cluster(int n);
+void nb_launch_build_cluster(const NbTreeBuffers& b, int n, int criterion, double theta, int drift,
+                             double dt, const double* shift, cudaStream_t s);
 void nb_launch_drift_only(NbTreeBuffers& b, int n, double dt, int numSMs, cudaStream_t s,
                           const double* shift = nullptr);
 // One half of the LMC's step (nb_lmc.cu): phase 0 drifts and kicks, phase 1 kicks; shift is
