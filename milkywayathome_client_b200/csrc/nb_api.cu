@@ -270,7 +270,7 @@ static NBodyCudaStatus nb_alloc_bodies(NBodyCudaState* st, int n)
     NB_CHECK(nb_alloc(&b.sort.idxA, N)); NB_CHECK(nb_alloc(&b.sort.idxB, N));
     const int tiles = (int) ((N + 2047) / 2048);
     NB_CHECK(nb_alloc(&b.sort.hist, 256 * (size_t) tiles));
-    NB_CHECK(nb_alloc(&b.sort.histTmp, (size_t) nb_scan_tmp_ints(256 * tiles)));
+    NB_CHECK(nb_alloc(&b.sort.histTmp, (size_t) std::max(256, nb_scan_tmp_ints(256 * tiles))));
     b.sort.capTiles = tiles;
     NB_CHECK(nb_alloc(&b.gx, N)); NB_CHECK(nb_alloc(&b.gy, N)); NB_CHECK(nb_alloc(&b.gz, N));
     NB_CHECK(nb_alloc(&b.delta, N)); NB_CHECK(nb_alloc(&b.cum, N));

@@ -260,7 +260,7 @@ __global__ void k_b_emit_bodies(const double* __restrict__ px, const double* __r
         maxLev = max(maxLev, lev);
     }
     for (int o = 16; o > 0; o >>= 1) maxLev = max(maxLev, __shfl_xor_sync(NB_FULL_MASK, maxLev, o));
-    if ((threadIdx.x & 31) == 0 && maxLev) atomicMax(&sc->maxDepth, maxLev);
+    nb_raise_max(&sc->maxDepth, maxLev);
 }
 
 // Cells owned by boundary a (as k_emit_cells), geometry from the dwarf's root size; the
@@ -386,7 +386,7 @@ int nb_build_forest(NbTreeBuffers& b, const NbForest& f, int n, int capNodes, in
                               b.sort.idxA, b.sc);
     launches += 4;
     nb_radix_sort_grouped(b.sort, n, f.bodyDwarf, s);
-    launches += 50;
+    launches += 30;
     k_b_gather_grid<<<g, T, 0, s>>>(b.px, b.py, b.pz, b.sort.idxA, f.bodyDwarf, f.dwarfs, b.gx,
                                     b.gy, b.gz, n, b.sc);
     k_b_fix_runs<<<g, T, 0, s>>>(b.sort.keyA, f.bodyDwarf, b.sort.idxA, b.gx, b.gy, b.gz, n, b.sc);
@@ -407,7 +407,7 @@ int nb_build_forest(NbTreeBuffers& b, const NbForest& f, int n, int capNodes, in
         b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.nodeRange, b.nodeQuad, b.parent, b.pending,
         b.cellNode, b.walkKids, f.bodyDwarf, f.dwarfs, criterion, theta, useQuad, b.sc);
     launches += 5;
-    nb_count_launch(launches - 53);       // the sort and the scan count their own
+    nb_count_launch(launches - 33);       // the sort and the scan count their own
     return launches;
 }
 

@@ -73,8 +73,14 @@ __global__ void k_keys(NbTreeBuffers b, int n, NbScalars* __restrict__ sc)
         b.sort.keyA[i] = k;
         b.sort.idxA[i] = (unsigned) i;
     }
+    // one atomic a block: they all go to one word, a few ns each
+    __shared__ int blockCount;
+    if (threadIdx.x == 0) blockCount = 0;
+    __syncthreads();
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(NB_FULL_MASK, cnt, o);
-    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(&sc->nTree, cnt);
+    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(&blockCount, cnt);
+    __syncthreads();
+    if (threadIdx.x == 0 && blockCount) atomicAdd(&sc->nTree, blockCount);
 }
 
 // Grid coordinates of the sorted bodies.
@@ -134,7 +140,7 @@ __global__ void k_emit_bodies(NbTreeBuffers b, NbScalars* __restrict__ sc)
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
         maxLev = max(maxLev, nb_phase_emit_body(b, i, m));
     for (int o = 16; o > 0; o >>= 1) maxLev = max(maxLev, __shfl_xor_sync(NB_FULL_MASK, maxLev, o));
-    if ((threadIdx.x & 31) == 0 && maxLev) atomicMax(&sc->maxDepth, maxLev);
+    nb_raise_max(&sc->maxDepth, maxLev);
 }
 
 __global__ void k_emit_cells(NbTreeBuffers b, int criterion, double theta, NbScalars* __restrict__ sc)
