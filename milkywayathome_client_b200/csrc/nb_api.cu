@@ -688,9 +688,8 @@ extern "C++" {
 // Large copies to pageable host memory: kStageSlots host threads, each with a page-locked slot of
 // the state, fetch a slot's worth from the device and move it into the caller's memory, in turn.
 // The driver's own staging moves it with one thread, which also takes the faults of fresh pages:
-// 4.5 GB/s for 30 MB arrays (8.2, 13.1 and 19.1 here for 10, 30 and 120 MB).  (Uploads gained nothing:
-// 18.8 GB/s by the driver, 12
-// staged.)  Below kStageMin the threads cost more than they save.
+// 4.5 GB/s for 30 MB arrays (8.2, 13.1 and 19.1 here for 10, 30 and 120 MB).  Uploads gained
+// nothing: 18.8 GB/s by the driver, 12 staged.  Below kStageMin the threads cost more than they save.
 static const int kStageSlots = 8;
 static const size_t kStageSlot = (size_t) 1 << 20;
 static const size_t kStageMin = (size_t) 4 << 20;

@@ -13,7 +13,7 @@
 // counting sort then lists the bodies of every bin in body order: one warp per chunk of bodies
 // (chunks never straddle a dwarf) counts its bins (k_bin_rows), one block turns the counts into
 // list offsets (k_bin_offsets), and the chunk warps place their bodies (k_bin_scatter, lanes
-// of one bin ranked in lane order).  Finally one thread per (quantity, dwarf, bin) walks its
+// of one bin ranked in lane order).  Finally one warp per (quantity, dwarf, bin) walks its
 // bin's list once per pass -- the initial sums and IterMax outlier passes, each followed by
 // nbCalcDisp -- adding in body order, as the reference does (k_disp_bins): the dispersions
 // and averages equal the reference's bit for bit.  Counts are integers and exact.
