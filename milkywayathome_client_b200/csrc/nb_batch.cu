@@ -353,6 +353,25 @@ k_b_moments(double4* nodePM, double* nodeCrit, const int2* nodeLink, const int* 
     if (structErr) nb_raise(sc, NBODY_TREE_STRUCTURE_ERROR);
 }
 
+// The same with eight lanes per cell.
+__global__ void __launch_bounds__(NB_MOM_WARPS * 32)
+k_b_moments_team(double4* nodePM, double* nodeCrit, const int2* nodeLink, const int* nodeDepth,
+            const int2* nodeRange, double* nodeQuad, const int* parent, int* pending,
+            const int* cellNode, const int4* kids, const int* __restrict__ bodyDwarf,
+            NbDwarfDev* dw, int criterion, double theta, int useQuad, NbScalars* sc)
+{
+    if (__any_sync(0xffffffffu, nb_failed(sc))) return;     // the lanes of a warp alike
+    bool structErr = false;
+    nb_moments_up(sc->nCells, nodePM, nodeCrit, nodeLink, nodeDepth, nodeRange, nodeQuad, parent,
+                  pending, cellNode, kids, criterion, theta, useQuad,
+                  [&](int first) { return dw[bodyDwarf[first]].rsize; },
+                  [&](int first) {
+                      structErr = true;
+                      atomicOr(&dw[bodyDwarf[first]].status, NBODY_TREE_STRUCTURE_ERROR);
+                  });
+    if (structErr) nb_raise(sc, NBODY_TREE_STRUCTURE_ERROR);
+}
+
 }  // namespace
 
 static inline int nb_b_grid(int n, int threads, int cap)
@@ -403,9 +422,14 @@ int nb_build_forest(NbTreeBuffers& b, const NbForest& f, int n, int capNodes, in
                                    b.sc);
     k_b_link_children<<<nb_b_grid(capNodes, T, 1 << 20), T, 0, s>>>(
         b.nodeLink, b.nodeDepth, b.nodeRange, b.parent, b.pending, b.cellNode, b.walkKids, b.sc);
-    k_b_moments<<<nb_b_grid(n, 128, 1 << 20), 128, 0, s>>>(
-        b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.nodeRange, b.nodeQuad, b.parent, b.pending,
-        b.cellNode, b.walkKids, f.bodyDwarf, f.dwarfs, criterion, theta, useQuad, b.sc);
+    if (nb_moments_team(n))
+        k_b_moments_team<<<nb_b_grid(n, NB_MOM_WARPS * 4, 1 << 20), NB_MOM_WARPS * 32, 0, s>>>(
+            b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.nodeRange, b.nodeQuad, b.parent,
+            b.pending, b.cellNode, b.walkKids, f.bodyDwarf, f.dwarfs, criterion, theta, useQuad, b.sc);
+    else
+        k_b_moments<<<nb_b_grid(n, 128, 1 << 20), 128, 0, s>>>(
+            b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.nodeRange, b.nodeQuad, b.parent,
+            b.pending, b.cellNode, b.walkKids, f.bodyDwarf, f.dwarfs, criterion, theta, useQuad, b.sc);
     launches += 5;
     nb_count_launch(launches - 33);       // the sort and the scan count their own
     return launches;

@@ -184,6 +184,22 @@ k_moments(double4* nodePM, double* nodeCrit, const int2* nodeLink, const int* no
     if (structErr) nb_raise(sc, NBODY_TREE_STRUCTURE_ERROR);
 }
 
+// Eight lanes per cell (nb_moments_up).
+__global__ void __launch_bounds__(NB_MOM_WARPS * 32)
+k_moments_team(double4* nodePM, double* nodeCrit, const int2* nodeLink, const int* nodeDepth,
+          const int2* nodeRange, double* nodeQuad, const int* parent, int* pending,
+          const int* cellNode, const int4* kids, int criterion, double theta, int useQuad,
+          NbScalars* sc)
+{
+    if (__any_sync(0xffffffffu, nb_failed(sc))) return;     // the lanes of a warp alike
+    const double rsize = sc->rsize;
+    bool structErr = false;
+    nb_moments_up(sc->nCells, nodePM, nodeCrit, nodeLink, nodeDepth, nodeRange, nodeQuad, parent,
+                  pending, cellNode, kids, criterion, theta, useQuad, [&](int) { return rsize; },
+                  [&](int) { structErr = true; });
+    if (structErr) nb_raise(sc, NBODY_TREE_STRUCTURE_ERROR);
+}
+
 // ---------------------------------------------------------------------------------
 // host driver
 // ---------------------------------------------------------------------------------
@@ -234,9 +250,14 @@ void nb_build_tree(NbTreeBuffers& b, int n, int capNodes, int criterion, double 
     else nb_launch_build_phases(b, n, capNodes, criterion, theta, drift, dt, numSMs, s, shift);
     // a cell parts at least two bodies (or is the root), but chains of single-child cells make
     // more of them than bodies now and then: the loop takes any number
-    k_moments<<<nb_grid_for(n, 128, 1 << 20), 128, 0, s>>>(
-        b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.nodeRange, b.nodeQuad, b.parent, b.pending,
-        b.cellNode, b.walkKids, criterion, theta, useQuad, b.sc);
+    if (nb_moments_team(n))
+        k_moments_team<<<nb_grid_for(n, NB_MOM_WARPS * 4, 1 << 20), NB_MOM_WARPS * 32, 0, s>>>(
+            b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.nodeRange, b.nodeQuad, b.parent,
+            b.pending, b.cellNode, b.walkKids, criterion, theta, useQuad, b.sc);
+    else
+        k_moments<<<nb_grid_for(n, 128, 1 << 20), 128, 0, s>>>(
+            b.nodePM, b.nodeCrit, b.nodeLink, b.nodeDepth, b.nodeRange, b.nodeQuad, b.parent,
+            b.pending, b.cellNode, b.walkKids, criterion, theta, useQuad, b.sc);
     nb_count_launch();
 }
 

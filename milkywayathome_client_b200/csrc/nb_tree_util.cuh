@@ -282,3 +282,142 @@ __device__ __forceinline__ void nb_bottom_up(int slot, const int* cellNode, cons
         __threadfence();
     }
 }
+
+// The same pass (nb_bottom_up over nb_cell_moments, the same operations in the same order) with
+// eight lanes a cell, where a chip that is not full waits for the chain of levels: each lane fetches
+// a child and computes its terms, and lane q adds quantity q of all eight through shared memory;
+// what is known of the parent (its children, centre and depth) is fetched meanwhile.  The four
+// cells of a warp go in step.  rsizeOf(first body) gives the root size of a start's tree,
+// outsideOf(first body) hears that a centre of mass left its cell.
+// The step outside the walk, a thread a cell -> eight lanes: 256 bodies 0.099 -> 0.075 ms, 1,024
+// 0.112 -> 0.093, 5,000 0.131 -> 0.108, 20,000 0.209 -> 0.184, 65,536 0.217 -> 0.202, 100,000
+// 0.230 -> 0.226; 262,144 0.306 -> 0.338, 1,048,576 0.689 -> 0.956, where issue slots are short and
+// most teams of a warp idle while one climbs: hence the line.
+constexpr int NB_MOM_WARPS = 4;
+constexpr int NB_MOM_TEAM_MAX = 100000;
+static inline bool nb_moments_team(int n) { return n <= NB_MOM_TEAM_MAX; }
+
+template <typename RsizeOf, typename OutsideOf>
+__device__ __forceinline__ void nb_moments_up(int nCells, double4* nodePM, double* nodeCrit,
+                                              const int2* __restrict__ nodeLink,
+                                              const int* __restrict__ nodeDepth,
+                                              const int2* __restrict__ nodeRange, double* nodeQuad,
+                                              const int* __restrict__ parent, int* pending,
+                                              const int* __restrict__ cellNode,
+                                              const int4* __restrict__ kids, int criterion,
+                                              double theta, int useQuad, RsizeOf rsizeOf,
+                                              OutsideOf outsideOf)
+{
+    const unsigned FULL = 0xffffffffu;
+    __shared__ __align__(16) double terms[NB_MOM_WARPS][4][6 * 8 + 8];  // + 8: teams in other banks
+    const int warp = threadIdx.x >> 5, team = (threadIdx.x & 31) >> 3, sub = threadIdx.x & 7;
+    double* const T = terms[warp][team];
+    const int* const kid8 = reinterpret_cast<const int*>(kids);
+    for (int base = (blockIdx.x * NB_MOM_WARPS + warp) * 4; base < nCells;
+         base += gridDim.x * NB_MOM_WARPS * 4) {
+        const int slot = base + team;
+        int c = slot < nCells ? cellNode[slot] : -1;    // complemented (< 0): waits for others
+        const int first = c - slot;                     // the cell's first body, as nb_link_cell
+        int kid = -1, D = 0;
+        bool kidCell = false;                           // a start has no child cells
+        double4 geo = make_double4(0.0, 0.0, 0.0, 0.0);
+        double rsize = 1.0;
+        if (c >= 0) {
+            kid = kid8[8 * (size_t) slot + sub];
+            D = nodeDepth[c];
+            geo = nb_ld_pm(&nodePM[c]);
+            rsize = rsizeOf(first);
+        }
+        while (__any_sync(FULL, c >= 0)) {
+            double4 q = make_double4(0.0, 0.0, 0.0, 0.0);
+            double2 A = make_double2(0.0, 0.0), B = A, C = A;
+            if (kid >= 0) q = nb_ld_pm(&nodePM[kid]);
+            if (kidCell && useQuad) {
+                const double2* kq = reinterpret_cast<const double2*>(nodeQuad + 6 * (size_t) kid);
+                A = __ldcg(kq); B = __ldcg(kq + 1); C = __ldcg(kq + 2);
+            }
+            const int p = c >= 0 ? parent[c] : -1;
+            T[sub] = q.w;                               // zeros past the last child: an ordered sum
+            T[8 + sub] = q.w * q.x;                     // from +0 is never -0, so they change nothing
+            T[16 + sub] = q.w * q.y;
+            T[24 + sub] = q.w * q.z;
+            int pFirst = 0, pD = 0;
+            double4 pGeo = geo;
+            if (p >= 0) {                               // (p's centre of mass waits for this cell)
+                pFirst = nodeRange[p].x;
+                pD = nodeDepth[p];
+                pGeo = nb_ld_pm(&nodePM[p]);
+            }
+            __syncwarp();
+            double s = 0.0;
+            const int row = sub & 3;
+#pragma unroll
+            for (int m = 0; m < 8; m += 2) {
+                const double2 t = *reinterpret_cast<const double2*>(&T[8 * row + m]);
+                s = s + t.x;
+                s = s + t.y;
+            }
+            const double M = __shfl_sync(FULL, s, 0, 8);
+            const double com = M > 0.0 ? s / M : row == 1 ? geo.x : row == 2 ? geo.y : geo.z;
+            const double cmx = __shfl_sync(FULL, com, 1, 8);
+            const double cmy = __shfl_sync(FULL, com, 2, 8);
+            const double cmz = __shfl_sync(FULL, com, 3, 8);
+            const int pKid = p >= 0 ? kid8[8 * (size_t) (p - pFirst) + sub] : -1;
+            double quad = 0.0;                          // of lanes 0 to 5
+            if (useQuad) {                              // else the record reads as zero
+                const double dx = q.x - cmx, dy = q.y - cmy, dz = q.z - cmz;
+                const double drsq = dz * dz + (dy * dy + dx * dx);
+                const double mq = q.w;
+                double txx = mq * (3.0 * (dx * dx) - drsq);
+                double txy = mq * (3.0 * (dx * dy));
+                double txz = mq * (3.0 * (dx * dz));
+                double tyy = mq * (3.0 * (dy * dy) - drsq);
+                double tyz = mq * (3.0 * (dy * dz));
+                double tzz = mq * (3.0 * (dz * dz) - drsq);
+                if (kidCell) {
+                    txx = txx + A.x; txy = txy + A.y; txz = txz + B.x;
+                    tyy = tyy + B.y; tyz = tyz + C.x; tzz = tzz + C.y;
+                }
+                if (kid < 0) txx = txy = txz = tyy = tyz = tzz = 0.0;
+                __syncwarp();                           // the sums above have been read
+                T[sub] = txx; T[8 + sub] = txy; T[16 + sub] = txz;
+                T[24 + sub] = tyy; T[32 + sub] = tyz; T[40 + sub] = tzz;
+                __syncwarp();
+                const int qrow = sub < 6 ? sub : 5;
+#pragma unroll
+                for (int m = 0; m < 8; m += 2) {
+                    const double2 t = *reinterpret_cast<const double2*>(&T[8 * qrow + m]);
+                    quad = quad + t.x;
+                    quad = quad + t.y;
+                }
+            }
+            const bool pKidCell = pKid >= 0 && nodeLink[pKid].y < 0;
+            if (c >= 0) {
+                const double psize = ldexp(rsize, -D);  // rsize halved D times: exact
+                const double h = 0.5 * psize;
+                const double crit = nb_find_rcrit2(criterion, theta, rsize, geo.x, geo.y, geo.z,
+                                                   cmx, cmy, cmz, psize);
+                if (sub < 6) nodeQuad[6 * (size_t) c + sub] = quad;
+                if (sub == 0) {
+                    nodeCrit[c] = crit;
+                    nodePM[c] = make_double4(cmx, cmy, cmz, M);
+                    if (cmx < geo.x - h || cmx > geo.x + h || cmy < geo.y - h ||
+                        cmy > geo.y + h || cmz < geo.z - h || cmz > geo.z + h)
+                        outsideOf(first);
+                }
+            }
+            __threadfence();                            // the cell, before its arrival
+            __syncwarp();                               // (and T is read before the next cell's terms)
+            int left = 0;
+            if (sub == 0 && p >= 0) left = atomicSub(&pending[p], 1);
+            left = __shfl_sync(FULL, left, 0, 8);
+            __threadfence();
+            const bool up = left == 1;
+            c = up ? p : -1;
+            kid = up ? pKid : -1;
+            kidCell = up && pKidCell;
+            D = pD;
+            geo = pGeo;
+        }
+    }
+}
