@@ -358,7 +358,7 @@ NBodyCudaStatus nbSetStepGraphCUDA(NBodyCudaState* st, int enable);
  * per-lane loads); 2 is the per-lane walk that loads the next node's record as soon as the opening
  * test has chosen it, overlapping that load with the current node's arithmetic (more registers:
  * faster for some tens of thousands of bodies, slower at a million).  -1 (the default) takes the
- * team walk up to 32,768 bodies; above, it cycles twice through forms 1 and 2 over a state's
+ * team walk up to 24,576 bodies (12,288 without quadrupoles); above, it cycles twice through forms 1 and 2 over a state's
  * first four uncounted FP64 tree evaluations, times the second round (the first launch of each
  * kernel also loads it) and keeps the faster.  Every form gives every body exactly its CPU walk --
  * same nodes, same order, same sums: the accelerations are the same bit for bit.  A batch takes
@@ -496,9 +496,9 @@ NBodyCudaStatus nbBatchSetTuningCUDA(NBodyCudaBatch* batch, int groupMax, int li
 /* as nbSetMixedModeCUDA, for every dwarf of the batch */
 NBodyCudaStatus nbBatchSetMixedModeCUDA(NBodyCudaBatch* batch, int exactSet);
 /* The FP64 walk's form for every dwarf of the batch, as nbSetWalkFormCUDA but without the
- * automatic choice: 0 (the default) the team walk for batches of up to 32,768 bodies in all and
- * per lane above, 1 per lane, 2 per lane with the next record loaded early (a warp may span two
- * dwarfs; each body walks only its own dwarf's tree). */
+ * choice by timing: 0 (the default) the form its bodies in all call for (the team walk up to 24,576,
+ * 12,288 without quadrupoles; then 2 up to 65,536, then 1), 1 per lane, 2 per lane with the next
+ * record loaded early (a warp may span two dwarfs; each body walks only its own dwarf's tree). */
 NBodyCudaStatus nbBatchSetWalkFormCUDA(NBodyCudaBatch* batch, int form);
 NBodyCudaStatus nbBatchGetTuningCUDA(NBodyCudaBatch* batch, int* groupMax, int* listCap,
                                      int* blocksPerSM);

@@ -185,7 +185,7 @@ struct NBodyCudaState {
     int useStepGraph = 1;
     int stepGraphForm = -1;
     NbScalars* scInit = nullptr;
-    // the FP64 walk's form (nbSetWalkFormCUDA): -1 takes the team walk where nb_walk_team(n) and
+    // the FP64 walk's form (nbSetWalkFormCUDA): -1 takes the team walk where nb_walk_team_auto and
     // chooses by timing above -- the first 2C uncounted FP64 tree evaluations cycle twice through
     // the C candidate forms, the second round (past each kernel's first launch, which also loads
     // it) is timed, the fastest form is kept
@@ -485,7 +485,7 @@ static NBodyCudaStatus nb_force(const NBodyCudaCtx* ctx, NBodyCudaState* st, int
     if (fp64Tree) {
         if (st->walkForm >= 0) form = st->walkForm;
         else if (st->walkFormChosen >= 0) form = st->walkFormChosen;
-        else if (nb_walk_team(n)) form = st->walkFormChosen = 0;
+        else if (nb_walk_team_auto(n, ctx->useQuad)) form = st->walkFormChosen = 0;
         else { form = kWalkTuneForms[st->walkTuneStep % kWalkTuneN]; tuning = !st->counting; }
     }
     // The device work of the evaluation, enqueued without host synchronisation: the scalars

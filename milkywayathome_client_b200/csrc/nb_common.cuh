@@ -312,9 +312,11 @@ size_t nb_mixed_stack_ints(int blocks);
 void nb_launch_pack_walk(const NbTreeBuffers& b, int capNodes, bool slots, cudaStream_t s);
 
 // The walks (forest != nullptr: one tree per dwarf, see NbForest).  form: the FP64 walk's
-// form, 0 the team walk where nb_walk_team(n) (else as 1), 1 the walk per lane, 2 per lane with
-// the next record loaded early.
+// form, 0 the team walk where nb_walk_team(n) (else as 1; of a forest the fastest by size), 1 the
+// walk per lane, 2 per lane with the next record loaded early.  nb_walk_team_auto: the sizes where
+// the team walk is the fastest form.
 bool nb_walk_team(int n);
+bool nb_walk_team_auto(int n, int useQuad);
 void nb_launch_walk_fp64(const NbTreeBuffers& b, int capNodes, const NbWalkParams& wp,
                          const NbPot& pot, bool count, cudaStream_t s,
                          const NbForest* forest = nullptr, int form = 0);

@@ -105,12 +105,18 @@ __device__ __forceinline__ void nb_radial(double s, double m, bool need, bool ce
 // opened cell, against ~190 a node for 32 bodies in the per-lane walk, which carries the
 // root-and-divisions chain of every node in its serial part on an eighth of the warps.  Five
 // resident blocks (96 registers): six to eight (80 to 64) were 3 to 20 % slower.
-// Walk times, per lane (the faster of its two forms, shared divisions) -> team, on the sampled
-// dwarf: 1,024 bodies (SW93, theta 1) 0.210 -> 0.106 ms, 5,000 (theta 1) 0.37 -> 0.155,
-// 20,000 (theta 1) 0.425 -> 0.333, (theta 0.5) 1.57 -> 1.07, 32,768 (theta 0.7) 0.861 -> 0.871,
-// 50,000 (theta 0.7) 0.996 -> 1.33.  Hence the line at TEAM_MAX_BODIES.
+// Walk times, per lane with the early load -> team, ms, on the two-component dwarf: with quadrupoles
+// 5,000 bodies (theta 1) 0.338 -> 0.159, 12,000 0.391 -> 0.213, 20,000 0.422 -> 0.349 (theta 0.5:
+// 1.457 -> 1.183), 25,000 0.430 -> 0.440 (0.7: 0.783 -> 0.774, 0.5: 1.537 -> 1.407), 32,768 0.461 ->
+// 0.542; without them, when the additions are most of a node's work, 5,000 0.190 -> 0.156, 12,000
+// 0.217 -> 0.211 (0.7: 0.362 -> 0.367, 0.5: 0.684 -> 0.713), 16,384 0.218 -> 0.306, 32,768 0.254 ->
+// 0.529.  Hence the automatic choice's two lines; form 0 asked for goes on to TEAM_MAX_BODIES.
 constexpr int TEAM_BODIES = 4;
 constexpr int TEAM_MAX_BODIES = 32768;
+constexpr int TEAM_AUTO_QUAD = 24576, TEAM_AUTO_MONO = 12288;
+// A batch past those lines: the early load while few warps are resident (20,000 bodies 0.497 ->
+// 0.422 ms, 32,768 0.534 -> 0.461; 1,048,576 7.41 -> 8.03).
+constexpr int EARLY_MAX_BODIES = 65536;
 constexpr int TEAM_LANES = 32 / TEAM_BODIES;                // 8: a cell's children
 constexpr unsigned TEAM_ALL = (1u << TEAM_BODIES) - 1u;     // every body of the warp
 constexpr unsigned TEAM_FIRST = 0x11111111u;                // the lanes with b = 0
@@ -722,6 +728,7 @@ void nb_launch_pack_walk(const NbTreeBuffers& b, int capNodes, bool slots, cudaS
 
 // The team walk below its line (form 0 is the per-lane walk above it).
 bool nb_walk_team(int n) { return n <= TEAM_MAX_BODIES; }
+bool nb_walk_team_auto(int n, int useQuad) { return n <= (useQuad ? TEAM_AUTO_QUAD : TEAM_AUTO_MONO); }
 
 void nb_launch_walk_fp64(const NbTreeBuffers& b, int capNodes, const NbWalkParams& wp,
                          const NbPot& pot, bool count, cudaStream_t s, const NbForest* forest,
@@ -732,6 +739,8 @@ void nb_launch_walk_fp64(const NbTreeBuffers& b, int capNodes, const NbWalkParam
     if (blocks <= 0) return;
     nb_launch_pack_walk(b, capNodes, true, s);
     const NbForest f = forest ? *forest : NbForest{nullptr, nullptr, 0};
+    if (forest && form == 0 && !nb_walk_team_auto(wp.n, wp.useQuad))
+        form = wp.n <= EARLY_MAX_BODIES ? 2 : 1;
     const bool team = form == 0 && nb_walk_team(wp.n);
     const int perTeamBlock = TEAM_BODIES * WALK_THREADS / 32;
     const int teamBlocks = (wp.n + perTeamBlock - 1) / perTeamBlock;

@@ -692,9 +692,8 @@ class NBodyBatch:
             self._h, int(group_max), int(list_cap), int(blocks_per_sm)))
 
     def set_walk_form(self, form=0):
-        """nbBatchSetWalkFormCUDA: the FP64 walk's form for every dwarf (0 the team walk for
-        batches of up to 32,768 bodies in all, 1 per lane, 2 per lane loading the next record
-        early); the accelerations are the same bit for bit."""
+        """nbBatchSetWalkFormCUDA: the FP64 walk's form for every dwarf (0 by the batch's
+        bodies in all, 1 per lane, 2 per lane loading the next record early); the accelerations are the same bit for bit."""
         self.check("nbBatchSetWalkFormCUDA", self.lib.nbBatchSetWalkFormCUDA(self._h, int(form)))
 
     def set_mixed_mode(self, exact=True):

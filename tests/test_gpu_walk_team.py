@@ -32,6 +32,20 @@ def test_small_sizes_equal_the_oracle(n, cfg):
     assert got_rc == rc and bits_equal(got, want)
 
 
+@pytest.mark.parametrize("n", [12288, 12289, 24576, 24577])
+@pytest.mark.parametrize("quad", [True, False])
+def test_the_automatic_choice_equals_every_form(n, quad):
+    """Both sides of its lines, with and without quadrupoles."""
+    from milkywayathome_client_b200 import models
+    pos, vel, mass, _ = models.plummer_plummer_dwarf(n, seed=6)
+    ctx = make_ctx(n, theta=0.9, useQuad=quad)
+    rc, want = _acc(ctx, pos, vel, mass, 1)
+    assert rc == 0
+    for form in (-1, 0, 2):
+        rc, got = _acc(ctx, pos, vel, mass, form)
+        assert rc == 0 and bits_equal(got, want), form
+
+
 @pytest.mark.parametrize("n", [32767, 32768, 32769])
 def test_both_sides_of_the_line_equal_the_per_lane_walk(n):
     from milkywayathome_client_b200 import models
