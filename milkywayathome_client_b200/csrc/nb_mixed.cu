@@ -15,7 +15,7 @@
 // centre ((hi - centre) + lo, formed once by the appending lane): the walk runs in coordinates
 // relative to the walking leaf group, so FP32 keeps its relative precision however far the
 // dwarf sits from the origin.  All 32 lanes then evaluate the list, each for its own body
-// (rsqrtf, explicit fmaf), and add the partial sums into FP64 after every cell list.  Centres
+// (nb_rsqrt, explicit fmaf), and add the partial sums into FP64 after every cell list.  Centres
 // of mass, moments, the external potential and the leapfrog stay FP64 (shared with the FP64
 // code, compiled with -fmad=false so the shared epilogue keeps the reference's rounding).
 #include "nb_common.cuh"
@@ -81,7 +81,7 @@ __global__ void k_pack_f32(const double4* __restrict__ nodePM, const double* __r
 // (explicit child lists built by k_pack_f32).  Popping from the top keeps the stack sorted by
 // depth, so at most 8 x 32 nodes of any one depth are ever on it: 256 x 63 levels bounds it
 // (NB_GROUP_STACK).  A full list is evaluated by all 32 lanes at once (each lane for its own
-// body, entries read as shared-memory broadcasts), FP32 with FMA and rsqrtf; partial sums go
+// body, entries read as shared-memory broadcasts), FP32 with FMA and nb_rsqrt; partial sums go
 // into FP64 accumulators after every list.  Persistent warps take groups from a counter.
 constexpr int GROUP_WARPS = 4;
 constexpr int GROUP_THREADS = 32 * GROUP_WARPS;
@@ -126,9 +126,8 @@ __device__ __forceinline__ void nb_acc_quad_if(unsigned tk, float sr, float dx, 
         : "r"(tk), "f"(sr), "f"(dx), "f"(dy), "f"(dz), "f"(ndr5), "f"(qx), "f"(qy), "f"(qz));
 }
 
-// 1/sqrt(x) of a normal x by the hardware's instruction (rsqrtf adds a scaling of subnormal
-// arguments to it: three instructions an interaction of ~40, and a squared distance that is
-// subnormal has an infinite attraction in FP32 either way).
+// 1/sqrt(x) by PTX's rsqrt.approx.ftz.f32, which takes a subnormal x as zero and returns infinity.
+// Walk at 1,048,576 bodies, rsqrtf -> this: 8.45 -> 7.53 ms (theta 0.5), 2.54 -> 2.30 (theta 1).
 __device__ __forceinline__ float nb_rsqrt(float x)
 {
     float y;
