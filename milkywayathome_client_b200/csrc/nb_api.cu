@@ -677,12 +677,14 @@ static NBodyCudaStatus nb_reset_run(NBodyCudaState* st, double treeRSize)
     return NBODY_SUCCESS;
 }
 
-static bool nb_is_pinned(const void* p)
+// Whether CUDA knows p as memory of this kind (cudaMemoryTypeUnregistered: pageable host memory).
+static bool nb_is_memory(const void* p, cudaMemoryType type)
 {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
-    return a.type == cudaMemoryTypeHost;
+    return a.type == type;
 }
+static bool nb_is_pinned(const void* p) { return nb_is_memory(p, cudaMemoryTypeHost); }
 
 extern "C++" {
 // Large copies to pageable host memory: kStageSlots host threads, each with a page-locked slot of
@@ -690,13 +692,15 @@ extern "C++" {
 // The driver's own staging moves it with one thread, which also takes the faults of fresh pages:
 // 4.5 GB/s for 30 MB arrays (8.2, 13.1 and 19.1 here for 10, 30 and 120 MB).  Uploads gained
 // nothing: 18.8 GB/s by the driver, 12 staged.  Below kStageMin the threads cost more than they save.
+// Every other kind of memory (page-locked, managed, a device pointer given by mistake) goes to
+// cudaMemcpyAsync, whose status the caller gets: a host thread must not write to what it cannot reach.
 static const int kStageSlots = 8;
 static const size_t kStageSlot = (size_t) 1 << 20;
 static const size_t kStageMin = (size_t) 4 << 20;
 
 static bool nb_stage_ready(NBodyCudaState* st, const void* host, size_t bytes)
 {
-    if (bytes < kStageMin || nb_is_pinned(host)) return false;
+    if (bytes < kStageMin || !nb_is_memory(host, cudaMemoryTypeUnregistered)) return false;
     if (st->hostStage) return true;
     for (cudaEvent_t& e : st->stageEv)
         if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
