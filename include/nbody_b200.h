@@ -358,13 +358,14 @@ NBodyCudaStatus nbSetStepGraphCUDA(NBodyCudaState* st, int enable);
  * per-lane loads); 2 is the per-lane walk that loads the next node's record as soon as the opening
  * test has chosen it, overlapping that load with the current node's arithmetic (more registers:
  * faster for some tens of thousands of bodies, slower at a million).  -1 (the default) takes the
- * team walk up to 24,576 bodies (12,288 without quadrupoles); above, it cycles twice through forms 1 and 2 over a state's
- * first four uncounted FP64 tree evaluations, times the second round (the first launch of each
- * kernel also loads it) and keeps the faster.  Every form gives every body exactly its CPU walk --
+ * team walk up to 24,576 bodies (12,288 without quadrupoles; decided at every evaluation); above,
+ * it cycles twice through forms 1 and 2 over a state's first four uncounted FP64 tree evaluations
+ * (with quadrupoles and without each by its own), times the second round (the first launch of
+ * each kernel also loads it) and keeps the faster.  Every form gives every body exactly its CPU walk --
  * same nodes, same order, same sums: the accelerations are the same bit for bit.  A batch takes
  * form 0 unless its form is set (nbBatchSetWalkFormCUDA); the force adjoint walks the union of a
  * warp's paths (it reduces each node's adjoints over the warp).
- * nbGetWalkFormCUDA reports the form in use (-1 before the first evaluation or while undecided). */
+ * nbGetWalkFormCUDA reports the last evaluation's form (-1 before the first and while undecided). */
 NBodyCudaStatus nbSetWalkFormCUDA(NBodyCudaState* st, int form);
 NBodyCudaStatus nbGetWalkFormCUDA(NBodyCudaState* st, int* form);
 

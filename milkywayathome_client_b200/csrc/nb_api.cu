@@ -185,14 +185,14 @@ struct NBodyCudaState {
     int useStepGraph = 1;
     int stepGraphForm = -1;
     NbScalars* scInit = nullptr;
-    // the FP64 walk's form (nbSetWalkFormCUDA): -1 takes the team walk where nb_walk_team_auto and
-    // chooses by timing above -- the first 2C uncounted FP64 tree evaluations cycle twice through
+    // the FP64 walk's form (nbSetWalkFormCUDA): -1 takes the team walk where nb_walk_team_auto (asked
+    // at every evaluation: it depends on the context) and chooses by timing above, with and without
+    // quadrupoles each by its own -- the first 2C uncounted FP64 tree evaluations cycle twice through
     // the C candidate forms, the second round (past each kernel's first launch, which also loads
     // it) is timed, the fastest form is kept
     int walkForm = -1;
-    int walkFormChosen = -1;
-    int walkTuneStep = 0;
-    float walkFormMs[8] = {-1.0f, -1.0f, -1.0f, -1.0f, -1.0f, -1.0f, -1.0f, -1.0f};
+    struct WalkTune { int step = 0, chosen = -1; float ms[kWalkTuneN] = {}; } walkTune[2];
+    int walkFormLast = -1;              // the last evaluation's, -1 while its choice is open
     char* hostStage = nullptr;          // page-locked staging of large copies (kStageSlots slots)
     cudaEvent_t stageEv[8] = {};        // each slot's copy from the device
     double* keepPos = nullptr;          // bodies at the best likelihood (3n each)
@@ -480,14 +480,17 @@ static NBodyCudaStatus nb_force(const NBodyCudaCtx* ctx, NBodyCudaState* st, int
     }
     // the FP64 walk's form for this evaluation (its timing decides the automatic choice)
     const bool fp64Tree = !mixed && ctx->criterion != NBCUDA_EXACT;
+    NBodyCudaState::WalkTune& tune = st->walkTune[ctx->useQuad ? 1 : 0];
     int form = 0;
-    bool tuning = false;
+    bool open = false;                  // the choice by timing is still to come
     if (fp64Tree) {
         if (st->walkForm >= 0) form = st->walkForm;
-        else if (st->walkFormChosen >= 0) form = st->walkFormChosen;
-        else if (nb_walk_team_auto(n, ctx->useQuad)) form = st->walkFormChosen = 0;
-        else { form = kWalkTuneForms[st->walkTuneStep % kWalkTuneN]; tuning = !st->counting; }
+        else if (nb_walk_team_auto(n, ctx->useQuad)) form = 0;
+        else if (tune.chosen >= 0) form = tune.chosen;
+        else { form = kWalkTuneForms[tune.step % kWalkTuneN]; open = true; }
+        st->walkFormLast = open ? -1 : form;
     }
+    const bool tuning = open && !st->counting;
     // The device work of the evaluation, enqueued without host synchronisation: the scalars
     // from the pinned st->scInit, the tree or the direct sum, the walk, the scalars back into
     // st->scHost.  capturing: inside a stream capture (events become graph nodes).
@@ -585,13 +588,12 @@ static NBodyCudaStatus nb_force(const NBodyCudaCtx* ctx, NBodyCudaState* st, int
         cudaEventElapsedTime(&ms, st->ev0, st->ev1);
         st->walkMs = ms;
         if (tuning && !(h.status & ~(int) NBODY_STATUS_WARNINGS_MASK)) {
-            const int c = st->walkTuneStep % kWalkTuneN;
-            if (st->walkTuneStep >= kWalkTuneN) st->walkFormMs[c] = ms;
-            if (++st->walkTuneStep == 2 * kWalkTuneN) {
+            tune.ms[tune.step % kWalkTuneN] = ms;
+            if (++tune.step == 2 * kWalkTuneN) {
                 int best = 0;
                 for (int k = 1; k < kWalkTuneN; ++k)
-                    if (st->walkFormMs[k] < st->walkFormMs[best]) best = k;
-                st->walkFormChosen = kWalkTuneForms[best];
+                    if (tune.ms[k] < tune.ms[best]) best = k;
+                st->walkFormLast = tune.chosen = kWalkTuneForms[best];
             }
         }
         ms = 0.0f;
@@ -1888,16 +1890,15 @@ NBodyCudaStatus nbSetWalkFormCUDA(NBodyCudaState* st, int form)
 {
     if (!st || form < -1 || form > 2) return NBODY_USER_ERROR;
     st->walkForm = form;
-    st->walkFormChosen = -1;
-    st->walkTuneStep = 0;
-    for (float& ms : st->walkFormMs) ms = -1.0f;
+    for (NBodyCudaState::WalkTune& t : st->walkTune) t = {};
+    st->walkFormLast = -1;
     return NBODY_SUCCESS;
 }
 
 NBodyCudaStatus nbGetWalkFormCUDA(NBodyCudaState* st, int* form)
 {
     if (!st || !form) return NBODY_USER_ERROR;
-    *form = st->walkForm >= 0 ? st->walkForm : st->walkFormChosen;
+    *form = st->walkForm >= 0 ? st->walkForm : st->walkFormLast;
     return NBODY_SUCCESS;
 }
 

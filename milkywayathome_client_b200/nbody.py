@@ -403,12 +403,12 @@ class NBodyState:
     def set_walk_form(self, form=-1):
         """The FP64 walk's form (nbSetWalkFormCUDA): 0 the team walk (up to 32,768 bodies; per
         lane above), 1 per lane, 2 per lane with the next node's record loaded early, -1 the
-        team walk or, above it, the faster of the other two by timing the first evaluations; the
-        accelerations are the same bit for bit."""
+        team walk up to 24,576 bodies (12,288 without quadrupoles) or, above, the faster of the
+        other two by timing the first evaluations; the accelerations are the same bit for bit."""
         self.check("nbSetWalkForm", self.lib.nbSetWalkFormCUDA(self._h, int(form)))
 
     def walk_form(self):
-        """The FP64 walk form in use (-1 while the automatic choice is undecided)."""
+        """The last FP64 tree evaluation's walk form (-1 while the automatic choice is undecided)."""
         f = ctypes.c_int()
         self.check("nbGetWalkForm", self.lib.nbGetWalkFormCUDA(self._h, ctypes.byref(f)))
         return f.value

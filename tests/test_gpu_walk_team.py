@@ -46,6 +46,24 @@ def test_the_automatic_choice_equals_every_form(n, quad):
         assert rc == 0 and bits_equal(got, want), form
 
 
+def test_the_automatic_choice_follows_the_context():
+    """A state's evaluations with and without quadrupoles each take the form of their own: the
+    team walk by its line (20,000 lies between the two), the timed choice kept for its kind."""
+    from milkywayathome_client_b200 import NBodyState, models
+    n = 20000
+    pos, vel, mass, _ = models.plummer_plummer_dwarf(n, seed=6)
+    quad, mono = make_ctx(n, theta=0.9), make_ctx(n, theta=0.9, useQuad=False)
+    with NBodyState.create(quad, pos, vel, mass, gravmap=False) as st:
+        assert st.walk_form() == -1
+        seen = []
+        for ctx in (quad, mono, mono, quad, mono, mono, quad, mono):
+            assert st.gravMap(ctx) == 0
+            seen.append(st.walk_form())
+        assert [seen[k] for k in (0, 3, 6)] == [0, 0, 0]
+        assert [seen[k] for k in (1, 2, 4)] == [-1, -1, -1]     # four evaluations decide
+        assert seen[5] in (1, 2) and seen[7] == seen[5]
+
+
 @pytest.mark.parametrize("n", [32767, 32768, 32769])
 def test_both_sides_of_the_line_equal_the_per_lane_walk(n):
     from milkywayathome_client_b200 import models
