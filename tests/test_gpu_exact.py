@@ -33,3 +33,27 @@ def test_operands_outside_the_shared_ranges(eps2, scale):
     with NBodyState.create(ctx, pos, vel, mass, gravmap=False) as st:
         assert st.gravMap(ctx) == rc
         assert np.array_equal(st.accels(), want, equal_nan=True)
+
+
+@pytest.mark.parametrize("criterion,form", [("Exact", 0), ("TreeCode", 0), ("TreeCode", 1)])
+def test_operands_next_to_midpoints(criterion, form):
+    """Two bodies so close that s = |dr|^2 + eps^2 is eps^2: the softened distances whose root or
+    reciprocal lies next to a midpoint of two doubles (tests/test_rdiv.py), with the device's own
+    reciprocal estimate."""
+    from milkywayathome_client_b200 import NBodyState
+    from test_rdiv import HARD_RECIPROCALS, hard_roots
+    d = 2.0 ** -30
+    pos, vel = np.array([[0.0, 0.0, 0.0], [d, 0.0, 0.0]]), np.zeros((2, 3))
+    rng = np.random.default_rng(1)
+    for s in hard_roots() + HARD_RECIPROCALS:
+        for k in (0, 1, 9):
+            eps2 = s * 4.0 ** k
+            mass = 1.0 + rng.integers(0, 1 << 52, 2) * 2.0 ** -52
+            ctx = make_ctx(2, criterion=criterion, theta=0.5, eps2=eps2, potential=None)
+            assert d * d + eps2 == eps2
+            with NBodyState.create(ctx, pos, vel, mass, gravmap=False) as st:
+                st.set_walk_form(form)
+                assert st.gravMap(ctx) == 0
+                acc = st.accels()
+            want = ((mass[::-1] / np.sqrt(eps2)) / eps2) * np.array([d, -d])
+            assert bits_equal(acc[:, 0], want) and not acc[:, 1:].any(), (s, k)

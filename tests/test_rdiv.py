@@ -9,6 +9,7 @@ roots and quotients constructed to lie next to a rounding boundary.
 import ctypes
 import os
 import subprocess
+from fractions import Fraction
 
 import numpy as np
 import pytest
@@ -31,6 +32,21 @@ extern "C" void radial(const double* s, const double* m, const double* a, int n,
         out[5 * i + 4] = nb_quot(a[i], s[i], z);
     }
 }
+extern "C" void reciprocals(const double* s, int n, double* out)
+{
+    for (int i = 0; i < n; ++i) {
+        double y;
+        const double r = nb_sqrt_recip(s[i], nb_rsqrt_estimate(s[i]), y);
+        out[4 * i] = r;
+        out[4 * i + 1] = y;                                 // nearly rounded 1 / r
+        out[4 * i + 2] = nb_recip_step(s[i], y * y);        // nearly rounded 1 / s
+        out[4 * i + 3] = nb_recip_step(s[i], out[4 * i + 2]);
+    }
+}
+extern "C" void quotients(const double* a, const double* b, const double* y, int n, double* out)
+{
+    for (int i = 0; i < n; ++i) out[i] = nb_quot(a[i], b[i], y[i]);
+}
 extern "C" void plummer(const double* s, const double* m, const double* x, const double* a, int n,
                         double* out)
 {
@@ -49,6 +65,32 @@ extern "C" void ranges(const double* x, int n, int* out)
                  nb_near_ones(x[i]) << 2;
 }
 '''
+
+
+# operands whose 1 / s, or whose root's reciprocal, one step from a few ulps does not round
+HARD_RECIPROCALS = [4663060627120798 * 2.0 ** -53, 8042426583074580 * 2.0 ** -53,
+                    float.fromhex("0x1.30a0dd90e13a2p+0"), float.fromhex("0x1.63baaac17d1e2p+1"),
+                    float.fromhex("0x1.0499b629293abp+0"), float.fromhex("0x1.0d5f392d40883p+0")]
+
+
+def hard_roots():
+    """Every s in [1, 4) whose root lies within 40 units of 2^-106 / (2 sqrt(s)) of a midpoint m of
+    two doubles: with M = 2^53 m odd, s = (M^2 - c) 2^-106 for |c| < 40 (c = 1 mod 8, for M^2 is and s
+    is a multiple of 2^-52).  The four roots of M^2 = c mod 2^k follow from those mod 2^(k - 1)."""
+    found = []
+    for c in range(-39, 40, 8):
+        for k, top in ((54, 2.0), (55, 4.0)):       # s below 2: multiples of 2^-52; below 4: of 2^-51
+            roots = {1, 3, 5, 7}
+            for j in range(4, k + 1):
+                roots = {r + h for r in roots for h in (0, 1 << (j - 1))
+                         if ((r + h) ** 2 - c) % (1 << j) == 0}
+            for M in roots:
+                if (1 << 53) < M < (1 << 54):
+                    s = (M * M - c) / 2.0 ** 106    # an integer of 53 bits times a power of two
+                    assert Fraction(s) == Fraction(M * M - c, 1 << 106) or not top / 2 <= s < top
+                    if top / 2 <= s < top:
+                        found.append(s)
+    return found
 
 
 @pytest.fixture(scope="module")
@@ -121,6 +163,78 @@ def test_operands_next_to_rounding_boundaries(lib):
                      np.nextafter(0.25, 0), np.nextafter(0.5, 1)])
     g = np.array(np.meshgrid(edge, edge, edge)).reshape(3, -1)
     _check(lib, *g)
+
+
+def test_hard_roots(lib):
+    """The only operands the bound on the root leaves open, in several binades."""
+    hard = hard_roots()
+    assert len(hard) >= 10 and 1.0 + 2.0 ** -52 in hard
+    s = np.array([h * 4.0 ** k for h in hard for k in (-50, -26, -3, 0, 1, 17, 49)])
+    _check(lib, s, np.ones_like(s), np.full_like(s, 3.0))
+
+
+def _off(y, b):
+    """|y - 1/b| in ulps of 1/b, exactly."""
+    inv = 1 / Fraction(b)
+    ulp = Fraction(2.0 ** np.floor(np.log2(float(inv)))) / 2 ** 52
+    while ulp * 2 ** 52 > inv:
+        ulp /= 2
+    while ulp * 2 ** 53 <= inv:
+        ulp *= 2
+    return abs(Fraction(y) - inv) / ulp
+
+
+def test_reciprocals_are_nearly_rounded(lib):
+    """What nb_quot and the second step are given: |y - 1/b| <= (1/2 + 2^-40) ulp, b the root and s;
+    a second step then rounds 1 / s.  On random operands and on those where one step does not."""
+    rng = np.random.default_rng(3)
+    s = np.concatenate([HARD_RECIPROCALS, hard_roots(), _random(rng, 4000, -100, 100)])
+    s = s[~_near_ones(s)]
+    out = np.empty((len(s), 4))
+    lib.reciprocals(s.ctypes.data_as(ctypes.c_void_p), ctypes.c_int(len(s)),
+                    out.ctypes.data_as(ctypes.c_void_p))
+    assert np.array_equal(out[:, 0], np.sqrt(s)) and np.array_equal(out[:, 3], 1.0 / s)
+    bound = Fraction(1, 2) + Fraction(1, 1 << 40)
+    for x, (r, y, z, _) in zip(s, out):
+        assert _off(y, r) <= bound and _off(z, x) <= bound
+    first = out[:len(HARD_RECIPROCALS)]
+    assert ((first[:, 2] != 1.0 / s[:len(first)]) | (first[:, 1] != 1.0 / first[:, 0])).any()
+
+
+def test_quotients_from_either_neighbour(lib):
+    """Quotients next to midpoints, divided with the worst nearly rounded reciprocals there are: of
+    divisors whose reciprocal lies next to a midpoint, both neighbours of it."""
+    rng = np.random.default_rng(4)
+    b = np.array(HARD_RECIPROCALS[:4])
+    out = np.empty((4, 4))
+    lib.reciprocals(b.ctypes.data_as(ctypes.c_void_p), ctypes.c_int(4),
+                    out.ctypes.data_as(ctypes.c_void_p))
+    bound = Fraction(1, 2) + Fraction(1, 1 << 40)
+    tried = 0
+    for x in b:
+        ys = [y for y in (np.nextafter(1.0 / x, 0), 1.0 / x, np.nextafter(1.0 / x, 9))
+              if _off(y, x) <= bound]
+        assert len(ys) == 2
+        X = int(np.ldexp(x, 53 - np.frexp(x)[1]))           # 53 bits
+        # midpoints M (odd, 54 bits): random ones, and those that put X M next to a double, by
+        # solving odd(X) M = j mod 2^54
+        inv = pow(X // (X & -X), -1, 1 << 54)
+        Ms = [int(k) * 2 + 1 for k in rng.integers(1 << 52, 1 << 53, 2000)]
+        Ms += [M for M in (inv * j % (1 << 54) for j in range(-4001, 4002, 2)) if M >> 53]
+        a = []
+        for M in Ms:
+            p = X * M
+            sh = p.bit_length() - 53
+            a += [float((p >> sh) + d) for d in (-1, 0, 1, 2)]
+        a = np.array(a)
+        for y in ys:
+            got = np.empty_like(a)
+            full = np.full_like(a, x), np.full_like(a, y)
+            lib.quotients(*[v.ctypes.data_as(ctypes.c_void_p) for v in (a, *full)],
+                          ctypes.c_int(len(a)), got.ctypes.data_as(ctypes.c_void_p))
+            assert np.array_equal(got, a / x)
+            tried += len(a)
+    assert tried > 100000
 
 
 @pytest.mark.parametrize("hi", [100, 400])
