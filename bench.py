@@ -91,10 +91,11 @@ def parse_args():
                     help="steps of the energy-drift run of both forms (0: skip)")
     ap.add_argument("--theta2", type=float, default=1.0,
                     help="second opening angle measured for both forms (0: skip)")
-    ap.add_argument("--walk-form", choices=["auto", "team", "lanes", "prefetch"],
+    ap.add_argument("--walk-form", choices=["auto", "team", "union", "lanes", "prefetch"],
                     default="auto",
-                    help="the FP64 walk: chosen by size and timing (default), team, per lane, or "
-                         "per lane loading the next record early")
+                    help="the FP64 walk: chosen by size and timing (default), shared by a warp's "
+                         "bodies (team: small systems, union: others; one form), per lane, or per "
+                         "lane loading the next record early")
     ap.add_argument("--profile", choices=["fp64", "mixed", "adjoint", "batch", "config0"],
                     help="profiling entry: build the dwarf, run two force evaluations, exit")
     return ap.parse_args()
@@ -507,7 +508,15 @@ def form_accuracy(pos, vel, mass, c_cfg, dev, seed=4096):
     return out
 
 
-WALK_FORM_NAMES = {0: "team", 1: "per lane", 2: "per lane, next record loaded early"}
+WALK_FORM_NAMES = {0: "shared (team or union)", 1: "per lane", 2: "per lane, next record loaded early"}
+
+
+def walk_kernel(form, n, theta):
+    """(kernel, entry of the traffic profile) of a walk form at this size: form 0 is the team walk
+    for small systems and the union of a warp's paths, in the per-lane kernel, for others."""
+    if form == 0 and (n <= 12288 or (n <= 32768 and theta >= 0.2)):
+        return "k_walk_fp64_team", "fp64_walk_team"
+    return "k_walk_fp64_lanes", "fp64_walk_union" if form == 0 else "fp64_walk_lanes"
 
 
 def settle_walk_form(st, c):
@@ -716,13 +725,13 @@ def run_ours(args, dist):
         try:
             with open(PROFILE_TRAFFIC) as f:
                 prof = json.load(f)
-            rec = prof["fp64_walk_lanes" if info.walkForm >= 1 else "fp64_walk_team"]
+            rec = prof[walk_kernel(info.walkForm, n, args.theta)[1]]
             per_body = rec["dram_bytes"] / rec["n_bodies"]
             traffic = per_body * n
         except (OSError, KeyError, ValueError):
             traffic = None
     roofline = {"bound": "fp64",
-                "kernel": "k_walk_fp64_lanes" if info.walkForm >= 1 else "k_walk_fp64_team",
+                "kernel": walk_kernel(info.walkForm, n, args.theta)[0],
                 "achieved": achieved,
                 "peak": peak64, "unit": "TFLOP/s", "frac": achieved / peak64,
                 "traffic": traffic,
@@ -892,7 +901,7 @@ def run_profile(args):
 def main():
     args = parse_args()
     global WALK_FORM
-    WALK_FORM = {"auto": -1, "team": 0, "lanes": 1, "prefetch": 2}[args.walk_form]
+    WALK_FORM = {"auto": -1, "team": 0, "union": 0, "lanes": 1, "prefetch": 2}[args.walk_form]
     if args.impl == "reference":
         # the reference arm is host-only: rank 0 runs it, other ranks exit without work
         os.environ.setdefault("WORLD_SIZE", "1")

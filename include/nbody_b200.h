@@ -352,19 +352,21 @@ NBodyCudaStatus nbSetStepCUDA(NBodyCudaState* st, int step);
  * arguments) and counted evaluations are always launched directly. */
 NBodyCudaStatus nbSetStepGraphCUDA(NBodyCudaState* st, int enable);
 
-/* The FP64 force walk's form: 0 is the team walk for systems of up to 32,768 bodies (a warp walks
- * for four bodies, eight lanes each evaluating the nodes of one body's path) and the per-lane walk
- * above; 1 walks every body's path in its own lane (a lane idles only once its walk is over;
- * per-lane loads); 2 is the per-lane walk that loads the next node's record as soon as the opening
- * test has chosen it, overlapping that load with the current node's arithmetic (more registers:
- * faster for some tens of thousands of bodies, slower at a million).  -1 (the default) takes the
- * team walk up to 24,576 bodies (12,288 without quadrupoles; decided at every evaluation); above,
- * it cycles twice through forms 1 and 2 over a state's first four uncounted FP64 tree evaluations
- * (with quadrupoles and without each by its own), times the second round (the first launch of
- * each kernel also loads it) and keeps the faster.  Every form gives every body exactly its CPU walk --
- * same nodes, same order, same sums: the accelerations are the same bit for bit.  A batch takes
- * form 0 unless its form is set (nbBatchSetWalkFormCUDA); the force adjoint walks the union of a
- * warp's paths (it reduces each node's adjoints over the warp).
+/* The FP64 force walk's form: 0 shares a warp's node visits -- the team walk (a warp walks for four
+ * bodies, eight lanes each evaluating the nodes of one body's path) for systems of up to 12,288
+ * bodies, and up to 32,768 at theta >= 0.2; else the union walk (a lane a body, the warp visiting
+ * the union of its bodies' paths).  1 walks every body's path in its own lane (a lane idles only
+ * once its walk is over; per-lane loads); 2 is the per-lane walk that loads the next node's record
+ * as soon as the opening test has chosen it, overlapping that load with the current node's
+ * arithmetic (more registers: faster for some tens of thousands of bodies, slower at a million).
+ * -1 (the default) takes the team walk up to 24,576 bodies (12,288 without quadrupoles) at theta >=
+ * 0.2, asked at every evaluation; else it cycles twice through forms 1 and 2 (and 0 at theta < 0.5)
+ * over a state's first four (six) uncounted FP64 tree evaluations, with quadrupoles and without and
+ * on both sides of theta 0.5 each by its own, times the second round (the first launch of each
+ * kernel also loads it) and keeps the fastest.  Every form gives every body exactly its CPU walk
+ * -- same nodes, same order, same sums: the accelerations are the same bit for bit.  A batch takes
+ * its form by rule unless it is set (nbBatchSetWalkFormCUDA); the force adjoint walks the union of
+ * a warp's paths (it reduces each node's adjoints over the warp).
  * nbGetWalkFormCUDA reports the last evaluation's form (-1 before the first and while undecided). */
 NBodyCudaStatus nbSetWalkFormCUDA(NBodyCudaState* st, int form);
 NBodyCudaStatus nbGetWalkFormCUDA(NBodyCudaState* st, int* form);
@@ -497,9 +499,9 @@ NBodyCudaStatus nbBatchSetTuningCUDA(NBodyCudaBatch* batch, int groupMax, int li
 /* as nbSetMixedModeCUDA, for every dwarf of the batch */
 NBodyCudaStatus nbBatchSetMixedModeCUDA(NBodyCudaBatch* batch, int exactSet);
 /* The FP64 walk's form for every dwarf of the batch, as nbSetWalkFormCUDA but without the
- * choice by timing: 0 (the default) the form its bodies in all call for (the team walk up to 24,576,
- * 12,288 without quadrupoles; then 2 up to 65,536, then 1), 1 per lane, 2 per lane with the next
- * record loaded early (a warp may span two dwarfs; each body walks only its own dwarf's tree). */
+ * choice by timing: 0 (the default) takes the team, union or either per-lane walk by a rule on the
+ * bodies in all, the bodies a dwarf and theta; 1 per lane, 2 per lane with the next record loaded
+ * early (a warp may span two dwarfs; each body walks only its own dwarf's tree). */
 NBodyCudaStatus nbBatchSetWalkFormCUDA(NBodyCudaBatch* batch, int form);
 NBodyCudaStatus nbBatchGetTuningCUDA(NBodyCudaBatch* batch, int* groupMax, int* listCap,
                                      int* blocksPerSM);

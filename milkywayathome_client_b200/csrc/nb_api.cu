@@ -130,10 +130,13 @@ struct NbSlot {
     double lmc[6] = {0, 0, 0, 0, 0, 0};   // the LMC's position and velocity (LMC runs)
 };
 
-// The FP64 walk forms the automatic choice times above the team walk's line (nbSetWalkFormCUDA):
-// 1 the walk per lane, 2 the walk per lane that loads the next node's record early.
-static const int kWalkTuneForms[] = {1, 2};
-static const int kWalkTuneN = (int) (sizeof kWalkTuneForms / sizeof kWalkTuneForms[0]);
+// The FP64 walk forms the automatic choice times (nbSetWalkFormCUDA): 1 the walk per lane, 2 the
+// walk per lane that loads the next node's record early and, below kWalkTuneTheta, 0 (the team or the
+// union walk; from there on it is behind the others: 262,144 bodies 7.29 against 7.00 ms, 50,000 2.70
+// against 1.89).
+static const int kWalkTuneForms[] = {1, 2, 0};
+static const int kWalkTuneMax = (int) (sizeof kWalkTuneForms / sizeof kWalkTuneForms[0]);
+static const double kWalkTuneTheta = 0.5;
 
 struct NBodyCudaState {
     int device = 0;
@@ -186,12 +189,12 @@ struct NBodyCudaState {
     int stepGraphForm = -1;
     NbScalars* scInit = nullptr;
     // the FP64 walk's form (nbSetWalkFormCUDA): -1 takes the team walk where nb_walk_team_auto (asked
-    // at every evaluation: it depends on the context) and chooses by timing above, with and without
-    // quadrupoles each by its own -- the first 2C uncounted FP64 tree evaluations cycle twice through
-    // the C candidate forms, the second round (past each kernel's first launch, which also loads
+    // at every evaluation: it depends on the context) and chooses by timing elsewhere, with and without
+    // quadrupoles and on both sides of kWalkTuneTheta each by its own -- the first 2C uncounted FP64
+    // tree evaluations cycle twice through the C candidate forms, the second round (past each kernel's first launch, which also loads
     // it) is timed, the fastest form is kept
     int walkForm = -1;
-    struct WalkTune { int step = 0, chosen = -1; float ms[kWalkTuneN] = {}; } walkTune[2];
+    struct WalkTune { int step = 0, chosen = -1; float ms[kWalkTuneMax] = {}; } walkTune[2][2];
     int walkFormLast = -1;              // the last evaluation's, -1 while its choice is open
     char* hostStage = nullptr;          // page-locked staging of large copies (kStageSlots slots)
     cudaEvent_t stageEv[8] = {};        // each slot's copy from the device
@@ -480,14 +483,16 @@ static NBodyCudaStatus nb_force(const NBodyCudaCtx* ctx, NBodyCudaState* st, int
     }
     // the FP64 walk's form for this evaluation (its timing decides the automatic choice)
     const bool fp64Tree = !mixed && ctx->criterion != NBCUDA_EXACT;
-    NBodyCudaState::WalkTune& tune = st->walkTune[ctx->useQuad ? 1 : 0];
+    const bool smallTheta = ctx->theta < kWalkTuneTheta;
+    NBodyCudaState::WalkTune& tune = st->walkTune[ctx->useQuad ? 1 : 0][smallTheta];
+    const int tuneN = smallTheta ? kWalkTuneMax : kWalkTuneMax - 1;
     int form = 0;
     bool open = false;                  // the choice by timing is still to come
     if (fp64Tree) {
         if (st->walkForm >= 0) form = st->walkForm;
-        else if (nb_walk_team_auto(n, ctx->useQuad)) form = 0;
+        else if (nb_walk_team_auto(n, ctx->useQuad, ctx->theta)) form = 0;
         else if (tune.chosen >= 0) form = tune.chosen;
-        else { form = kWalkTuneForms[tune.step % kWalkTuneN]; open = true; }
+        else { form = kWalkTuneForms[tune.step % tuneN]; open = true; }
         st->walkFormLast = open ? -1 : form;
     }
     const bool tuning = open && !st->counting;
@@ -518,7 +523,8 @@ static NBodyCudaStatus nb_force(const NBodyCudaCtx* ctx, NBodyCudaState* st, int
                 nb_launch_walk_mixed(b, st->mx, st->capNodes, wp, pot, st->counting != 0,
                                      st->numSMs, s);
             else
-                nb_launch_walk_fp64(b, st->capNodes, wp, pot, st->counting != 0, s, nullptr, form);
+                nb_launch_walk_fp64(b, st->capNodes, wp, pot, st->counting != 0, s, nullptr,
+                                    form ? form : nb_walk_shared(n, ctx->theta));
             rec(st->ev1);
         }
         rec(st->evE);
@@ -588,10 +594,10 @@ static NBodyCudaStatus nb_force(const NBodyCudaCtx* ctx, NBodyCudaState* st, int
         cudaEventElapsedTime(&ms, st->ev0, st->ev1);
         st->walkMs = ms;
         if (tuning && !(h.status & ~(int) NBODY_STATUS_WARNINGS_MASK)) {
-            tune.ms[tune.step % kWalkTuneN] = ms;
-            if (++tune.step == 2 * kWalkTuneN) {
+            tune.ms[tune.step % tuneN] = ms;
+            if (++tune.step == 2 * tuneN) {
                 int best = 0;
-                for (int k = 1; k < kWalkTuneN; ++k)
+                for (int k = 1; k < tuneN; ++k)
                     if (tune.ms[k] < tune.ms[best]) best = k;
                 st->walkFormLast = tune.chosen = kWalkTuneForms[best];
             }
@@ -1890,7 +1896,8 @@ NBodyCudaStatus nbSetWalkFormCUDA(NBodyCudaState* st, int form)
 {
     if (!st || form < -1 || form > 2) return NBODY_USER_ERROR;
     st->walkForm = form;
-    for (NBodyCudaState::WalkTune& t : st->walkTune) t = {};
+    for (auto& row : st->walkTune)
+        for (NBodyCudaState::WalkTune& t : row) t = {};
     st->walkFormLast = -1;
     return NBODY_SUCCESS;
 }
@@ -2171,8 +2178,9 @@ static int nb_batch_enqueue(NBodyCudaBatch* bt, const NBodyCudaCtx* ctx, int dri
         nb_launch_walk_mixed(b, st->mx, st->capNodes, wp, pot, false, st->numSMs, s, &f);
         launches += 3;
     } else {
-        nb_launch_walk_fp64(b, st->capNodes, wp, pot, false, s, &f,
-                            st->walkForm > 0 ? st->walkForm : 0);
+        const int kernel = st->walkForm > 0 ? st->walkForm
+                                            : nb_walk_batch(st->nbody, bt->nDwarfs, ctx->useQuad, ctx->theta);
+        nb_launch_walk_fp64(b, st->capNodes, wp, pot, false, s, &f, kernel);
         launches += 1;
     }
     cudaEventRecord(st->ev1, s);

@@ -311,15 +311,18 @@ size_t nb_mixed_stack_ints(int blocks);
 // carry their slot in walkKids (the force adjoint's restored trees have none, and no use for it).
 void nb_launch_pack_walk(const NbTreeBuffers& b, int capNodes, bool slots, cudaStream_t s);
 
-// The walks (forest != nullptr: one tree per dwarf, see NbForest).  form: the FP64 walk's
-// form, 0 the team walk where nb_walk_team(n) (else as 1; of a forest the fastest by size), 1 the
-// walk per lane, 2 per lane with the next record loaded early.  nb_walk_team_auto: the sizes where
-// the team walk is the fastest form.
-bool nb_walk_team(int n);
-bool nb_walk_team_auto(int n, int useQuad);
+// The walks (forest != nullptr: one tree per dwarf, see NbForest).  The FP64 walk's kernels: the team
+// walk, per lane on its own path, the same with the next record loaded early, per lane on the
+// warp's union of paths.  nb_walk_shared: the kernel of form 0 (nbSetWalkFormCUDA); forms 1 and 2 are
+// NB_WALK_LANES and NB_WALK_EARLY.  nb_walk_team_auto: where the team walk is taken without timing.
+// nb_walk_batch: a batch's kernel by rule, of n bodies in all.
+enum { NB_WALK_TEAM = 0, NB_WALK_LANES = 1, NB_WALK_EARLY = 2, NB_WALK_UNION = 3 };
+int nb_walk_shared(int n, double theta);
+bool nb_walk_team_auto(int n, int useQuad, double theta);
+int nb_walk_batch(int n, int dwarfs, int useQuad, double theta);
 void nb_launch_walk_fp64(const NbTreeBuffers& b, int capNodes, const NbWalkParams& wp,
                          const NbPot& pot, bool count, cudaStream_t s,
-                         const NbForest* forest = nullptr, int form = 0);
+                         const NbForest* forest, int kernel);
 void nb_launch_walk_mixed(const NbTreeBuffers& b, const NbMixedBuffers& m, int capNodes,
                           const NbWalkParams& wp, const NbPot& pot, bool count, int numSMs,
                           cudaStream_t s, const NbForest* forest = nullptr);

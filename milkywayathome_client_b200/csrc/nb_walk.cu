@@ -6,9 +6,10 @@
 // At node q the body accepts (interacts, then jumps to Next(q)) if q is a body or |dr|^2 >=
 // rcrit2(q), otherwise it opens q (goes to More(q) = q + 1 in walk order).  Two kernels: the team
 // walk (k_walk_fp64_team) gives four bodies a warp and evaluates eight nodes at once for each, for
-// systems too small to fill the GPU with one lane a body; the per-lane walk (k_walk_fp64_lanes)
-// lets each lane walk its own body's path.  Either way each body gets exactly the nodes of its
-// own CPU walk, and sums the same terms in the CPU's order.  A monopole interaction is 18 flops
+// systems too small to fill the GPU with one lane a body; the walk with a lane a body
+// (k_walk_fp64_lanes), where each lane takes its own body's path, or the warp the union of its
+// bodies' paths.  Either way each body gets exactly the nodes of its own CPU walk, and sums the
+// same terms in the CPU's order.  A monopole interaction is 18 flops
 // + sqrt + 2 divisions, a quadrupole cell adds 38 flops + 2 divisions.
 #include "nb_common.cuh"
 #include "nb_potential.cuh"
@@ -110,13 +111,14 @@ __device__ __forceinline__ void nb_radial(double s, double m, bool need, bool ce
 // 1.457 -> 1.183), 25,000 0.430 -> 0.440 (0.7: 0.783 -> 0.774, 0.5: 1.537 -> 1.407), 32,768 0.461 ->
 // 0.542; without them, when the additions are most of a node's work, 5,000 0.190 -> 0.156, 12,000
 // 0.217 -> 0.211 (0.7: 0.362 -> 0.367, 0.5: 0.684 -> 0.713), 16,384 0.218 -> 0.306, 32,768 0.254 ->
-// 0.529.  Hence the automatic choice's two lines; form 0 asked for goes on to TEAM_MAX_BODIES.
+// 0.529.  Hence the automatic choice's two lines.  Small opening angles take few cells and many
+// bodies, whose work is mostly the additions again: quadrupoles, 24,000 bodies, union -> team: theta
+// 0.2 8.23 -> 7.85, 0.1 12.1 -> 15.7, 0.05 12.1 -> 20.4; 12,000: 0.1 5.94 -> 5.12, 0 7.09 -> 11.8.  So
+// form 0 is the team walk up to the smaller line, and up to TEAM_MAX_BODIES from TEAM_THETA on.
 constexpr int TEAM_BODIES = 4;
 constexpr int TEAM_MAX_BODIES = 32768;
 constexpr int TEAM_AUTO_QUAD = 24576, TEAM_AUTO_MONO = 12288;
-// A batch past those lines: the early load while few warps are resident (20,000 bodies 0.497 ->
-// 0.422 ms, 32,768 0.534 -> 0.461; 1,048,576 7.41 -> 8.03).
-constexpr int EARLY_MAX_BODIES = 65536;
+constexpr double TEAM_THETA = 0.2;
 constexpr int TEAM_LANES = 32 / TEAM_BODIES;                // 8: a cell's children
 constexpr unsigned TEAM_ALL = (1u << TEAM_BODIES) - 1u;     // every body of the warp
 constexpr unsigned TEAM_FIRST = 0x11111111u;                // the lanes with b = 0
@@ -324,7 +326,7 @@ k_walk_fp64_team(const double4* __restrict__ rec, const int* __restrict__ kids,
     if (p < 3) (p == 0 ? ax : p == 1 ? ay : az)[j] = acc;
 }
 
-// The walk with every lane on its own path: each iteration every lane
+// The walk with a lane a body.  LANES_OWN: each iteration every lane
 // that has not finished takes the next node of its own walk (a per-lane gather of the node
 // record, one 32-byte load per sector), so a lane is idle only when its walk is over.  Each lane
 // meets exactly its CPU walk's nodes in the CPU's order and sums the same terms in the same
@@ -334,7 +336,16 @@ k_walk_fp64_team(const double4* __restrict__ rec, const int* __restrict__ kids,
 // wavefronts a warp, more with distinct records) and the FP64 pipe (63 %).  Sharing one
 // reciprocal among the root and the divisions (nb_radial) took the 1,048,576-body dwarf from 28.9
 // to 28.1 ms at theta 0.5 and from 7.05 to 6.54 ms at theta 1.
-template <bool COUNT, bool FOREST, bool PREFETCH>
+// LANES_EARLY: the next node's record is loaded as soon as the opening test has chosen it, before
+// this node's terms are computed, so its latency overlaps the FP64 arithmetic (79 registers
+// against 63: it pays where few warps are resident, up to some 80,000 bodies).
+// LANES_UNION: the warp takes the smallest of its lanes' next nodes, the lanes that are at it do it:
+// one broadcast load a node, but an iteration for every node that any lane visits.  The smaller the
+// opening angle, the more of a walk its neighbours share: walks of 1,048,576 bodies, own -> union:
+// theta 0.7 12.4 -> 13.6 ms, 0.5 28.1 -> 28.2, 0.4 49.4 -> 44.2, 0.3 107 -> 84.5, 0.2 302 -> 210; 50,000
+// bodies, early -> union: 0.5 1.89 -> 2.70, 0.25 9.64 -> 9.98, 0.2 15.2 -> 13.6, 0.1 34.2 -> 22.3.
+enum { LANES_OWN, LANES_EARLY, LANES_UNION };
+template <bool COUNT, bool FOREST, int PATH>
 __global__ void __launch_bounds__(WALK_THREADS)
 k_walk_fp64_lanes(const double4* __restrict__ rec,
                   const unsigned int* __restrict__ order, const double* __restrict__ px,
@@ -364,10 +375,7 @@ k_walk_fp64_lanes(const double4* __restrict__ rec,
     double accx = 0.0, accy = 0.0, accz = 0.0;
     bool metSelf = false;
     unsigned long long cVisit = 0, cBB = 0, cBC = 0, cSteps = 0;
-    // PREFETCH: the next node's record is loaded as soon as the opening test has chosen it,
-    // before this node's terms are computed, so its latency overlaps the FP64 arithmetic (72
-    // registers against 56: it pays where few warps are resident, tens of thousands of bodies,
-    // and costs at a million, where other warps already hide the latency)
+    constexpr bool PREFETCH = PATH == LANES_EARLY;
     double4 nd = make_double4(0.0, 0.0, 0.0, 0.0), r1 = nd;
     if (PREFETCH && ptr < myEnd) {
         nd = nb_ld32(rec + 3 * (size_t) ptr);
@@ -376,11 +384,19 @@ k_walk_fp64_lanes(const double4* __restrict__ rec,
     for (;;) {
         // every lane takes part in the vote of every iteration (a finished lane idles in the
         // loop), and the warp leaves the loop together when all its walks are over
-        const bool active = ptr < myEnd;
-        if (!__any_sync(NB_FULL_MASK, active)) break;
+        int q = ptr;
+        bool active;
+        if (PATH == LANES_UNION) {
+            if (FOREST && ptr >= myEnd) ptr = end;      // this lane's tree is done
+            q = __reduce_min_sync(NB_FULL_MASK, ptr);
+            if (q >= end) break;
+            active = ptr == q;
+        } else {
+            active = ptr < myEnd;
+            if (!__any_sync(NB_FULL_MASK, active)) break;
+        }
         if (COUNT) ++cSteps;
         if (!active) continue;
-        const int q = ptr;
         if (!PREFETCH) {
             nd = nb_ld32(rec + 3 * (size_t) q);
             r1 = nb_ld32(rec + 3 * (size_t) q + 1);
@@ -726,22 +742,62 @@ void nb_launch_pack_walk(const NbTreeBuffers& b, int capNodes, bool slots, cudaS
     nb_count_launch();
 }
 
-// The team walk below its line (form 0 is the per-lane walk above it).
-bool nb_walk_team(int n) { return n <= TEAM_MAX_BODIES; }
-bool nb_walk_team_auto(int n, int useQuad) { return n <= (useQuad ? TEAM_AUTO_QUAD : TEAM_AUTO_MONO); }
+// Form 0's kernel, and where it is the team walk and the fastest form without timing.
+int nb_walk_shared(int n, double theta)
+{
+    return n <= TEAM_AUTO_MONO || (n <= TEAM_MAX_BODIES && theta >= TEAM_THETA) ? NB_WALK_TEAM
+                                                                               : NB_WALK_UNION;
+}
+bool nb_walk_team_auto(int n, int useQuad, double theta)
+{
+    return n <= (useQuad ? TEAM_AUTO_QUAD : TEAM_AUTO_MONO) && theta >= TEAM_THETA;
+}
+
+// A batch's kernel.  Its bodies in all fill the chip, but a body meets only those of its dwarf, of
+// which a small dwarf's walk takes most whatever the angle.  Measured: steps of batches of 40,000 to
+// 3,000,000 bodies in dwarfs of 200 to 100,000.
+//   * The team walk at sizes that leave the chip idle, as for single systems, but not where nearly
+//     every body is met: between its lines it needs bodies-a-dwarf x theta^2 >= 300 (20,000 bodies
+//     in all, early load -> team: 100 dwarfs, theta 1 0.310 -> 0.332 ms; 20, 1 0.440 -> 0.436, 0.5 0.687 ->
+//     0.705; 10, 0.5 0.926 -> 0.895, 0.2 1.39 -> 1.70; 2, 0.2 5.19 -> 4.76, 0.05 6.37 -> 8.76).
+//   * The union where walks share most of their nodes: theta^5 x bodies-a-dwarf <= 440 with a full
+//     chip (own path -> union: 20 dwarfs of 10,000, theta 0.6 3.14 -> 3.24, 0.5 4.36 -> 4.01, 0.3 10.2 ->
+//     7.20; 100 of 2,000, 0.85 1.34 -> 1.37, 0.7 1.66 -> 1.59, 0.5 2.44 -> 2.02), 990 from 524,288 bodies in
+//     all (1,000 of 1,000: 1.0 3.39 -> 3.58, 0.85 3.89 -> 3.86, 0.5 6.17 -> 5.06; 100 of 10,000: 0.7 8.72 ->
+//     8.96, 0.6 11.6 -> 11.4; 16 of 64,000: 0.5 22.6 -> 22.2, 0.4 37.1 -> 32.8), less below 131,072,
+//     where the longer walk's latency shows (early load -> union: 40 of 1,000, 0.7 0.596 -> 0.613, 0.5
+//     0.746 -> 0.709; 1 of 40,000, 0.3 5.8 -> 7.1), and less without quadrupoles (own path -> union: 20
+//     of 10,000, 0.5 2.84 -> 2.87, 0.4 4.22 -> 3.77; 100 of 10,000, 0.7 5.70 -> 6.30, 0.5 10.6 -> 10.3).
+//     Not where a walk is nearly all bodies (early load -> union: 50 dwarfs of 1,000, 0.1 0.907 -> 1.18)
+//     nor for the smallest dwarfs (200 of 200: 0.5 0.361 -> 0.430).
+//   * Else own paths, with the early load while few warps are resident (own -> early, theta 0.7: 65,536
+//     bodies 1.04 -> 0.97, 80,000 1.11 -> 1.04, 96,758 1.19 -> 1.20, 131,072 1.33 -> 1.57).
+constexpr int EARLY_MAX_BODIES = 81920;
+constexpr int UNION_FULL_BODIES = 131072, UNION_MANY_BODIES = 524288;
+int nb_walk_batch(int n, int dwarfs, int useQuad, double theta)
+{
+    const double mean = (double) n / dwarfs, cells = mean * (theta * theta);
+    if (n <= TEAM_AUTO_MONO && theta >= 0.02) return NB_WALK_TEAM;
+    if (useQuad && n <= TEAM_AUTO_QUAD && cells >= 300.0) return NB_WALK_TEAM;
+    const double full = n < UNION_FULL_BODIES ? (double) n / UNION_FULL_BODIES : 1.0;
+    const double shared = (theta * theta) * (theta * cells);
+    const bool many = n >= UNION_MANY_BODIES;
+    const double limit = useQuad ? (many ? 990.0 : 440.0 * (full * full))
+                                 : (many ? 1040.0 : full >= 0.75 ? 104.0 * (full * full) : -1.0);
+    if (mean >= 400.0 && cells * full >= 8.0 && shared <= limit && (useQuad || theta <= 0.5))
+        return NB_WALK_UNION;
+    return n <= EARLY_MAX_BODIES ? NB_WALK_EARLY : NB_WALK_LANES;
+}
 
 void nb_launch_walk_fp64(const NbTreeBuffers& b, int capNodes, const NbWalkParams& wp,
                          const NbPot& pot, bool count, cudaStream_t s, const NbForest* forest,
-                         int form)
+                         int kernel)
 {
     const int warps = (wp.n + 31) / 32;
     const int blocks = (warps * 32 + WALK_THREADS - 1) / WALK_THREADS;
     if (blocks <= 0) return;
     nb_launch_pack_walk(b, capNodes, true, s);
     const NbForest f = forest ? *forest : NbForest{nullptr, nullptr, 0};
-    if (forest && form == 0 && !nb_walk_team_auto(wp.n, wp.useQuad))
-        form = wp.n <= EARLY_MAX_BODIES ? 2 : 1;
-    const bool team = form == 0 && nb_walk_team(wp.n);
     const int perTeamBlock = TEAM_BODIES * WALK_THREADS / 32;
     const int teamBlocks = (wp.n + perTeamBlock - 1) / perTeamBlock;
 #define NB_LANES_ARGS b.walkRec, b.sort.idxA, b.px, b.py, b.pz, b.ax, b.ay, b.az, wp, b.sc, f
@@ -752,27 +808,22 @@ void nb_launch_walk_fp64(const NbTreeBuffers& b, int capNodes, const NbWalkParam
         if (count) k_walk_fp64_team<true, FOREST><<<teamBlocks, WALK_THREADS, 0, s>>>(NB_TEAM_ARGS); \
         else k_walk_fp64_team<false, FOREST><<<teamBlocks, WALK_THREADS, 0, s>>>(NB_TEAM_ARGS);    \
     } while (0)
-    if (forest) {
-        if (form == 2) {
-            if (count) k_walk_fp64_lanes<true, true, true><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
-            else k_walk_fp64_lanes<false, true, true><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
-        } else if (form == 1 || !team) {
-            if (count) k_walk_fp64_lanes<true, true, false><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
-            else k_walk_fp64_lanes<false, true, false><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
-        } else {
-            NB_TEAM(true);
-        }
-    } else {
-        if (form == 2) {
-            if (count) k_walk_fp64_lanes<true, false, true><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
-            else k_walk_fp64_lanes<false, false, true><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
-        } else if (form == 1 || !team) {
-            if (count) k_walk_fp64_lanes<true, false, false><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
-            else k_walk_fp64_lanes<false, false, false><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);
-        } else {
-            NB_TEAM(false);
-        }
-    }
+#define NB_LANES(FOREST, PATH)                                                                \
+    do {                                                                                      \
+        if (count) k_walk_fp64_lanes<true, FOREST, PATH><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS); \
+        else k_walk_fp64_lanes<false, FOREST, PATH><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);    \
+    } while (0)
+#define NB_WALK(FOREST)                                                                       \
+    do {                                                                                      \
+        if (kernel == NB_WALK_TEAM) NB_TEAM(FOREST);                                          \
+        else if (kernel == NB_WALK_EARLY) NB_LANES(FOREST, LANES_EARLY);                      \
+        else if (kernel == NB_WALK_UNION) NB_LANES(FOREST, LANES_UNION);                      \
+        else NB_LANES(FOREST, LANES_OWN);                                                     \
+    } while (0)
+    if (forest) NB_WALK(true);
+    else NB_WALK(false);
+#undef NB_WALK
+#undef NB_LANES
 #undef NB_TEAM
 #undef NB_LANES_ARGS
 #undef NB_TEAM_ARGS

@@ -401,10 +401,10 @@ class NBodyState:
                                                                   float(previous_forward_time)))
 
     def set_walk_form(self, form=-1):
-        """The FP64 walk's form (nbSetWalkFormCUDA): 0 the team walk (up to 32,768 bodies; per
-        lane above), 1 per lane, 2 per lane with the next node's record loaded early, -1 the
-        team walk up to 24,576 bodies (12,288 without quadrupoles) or, above, the faster of the
-        other two by timing the first evaluations; the accelerations are the same bit for bit."""
+        """The FP64 walk's form (nbSetWalkFormCUDA): 0 shares a warp's node visits (the team walk
+        for small systems, else the union of the warp's paths), 1 per lane, 2 per lane with the
+        next node's record loaded early, -1 the team walk where it is known to be the fastest, else
+        the fastest by timing the first evaluations; the accelerations are the same bit for bit."""
         self.check("nbSetWalkForm", self.lib.nbSetWalkFormCUDA(self._h, int(form)))
 
     def walk_form(self):
@@ -692,8 +692,9 @@ class NBodyBatch:
             self._h, int(group_max), int(list_cap), int(blocks_per_sm)))
 
     def set_walk_form(self, form=0):
-        """nbBatchSetWalkFormCUDA: the FP64 walk's form for every dwarf (0 by the batch's
-        bodies in all, 1 per lane, 2 per lane loading the next record early); the accelerations are the same bit for bit."""
+        """nbBatchSetWalkFormCUDA: the FP64 walk's form for every dwarf (0 by a rule on the batch's
+        sizes and theta, 1 per lane, 2 per lane loading the next record early); the accelerations
+        are the same bit for bit."""
         self.check("nbBatchSetWalkFormCUDA", self.lib.nbBatchSetWalkFormCUDA(self._h, int(form)))
 
     def set_mixed_mode(self, exact=True):

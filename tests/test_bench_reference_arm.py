@@ -99,3 +99,6 @@ def test_walk_form_is_settled_before_timed_steps():
     bench.settle_walk_form(st, ctx.with_precision("mixed"))
     assert st.evaluations == 0
     assert set(bench.WALK_FORM_NAMES) == {0, 1, 2}
+    assert bench.walk_kernel(0, 20000, 1.0)[0] == "k_walk_fp64_team"
+    assert bench.walk_kernel(0, 1048576, 0.5) == ("k_walk_fp64_lanes", "fp64_walk_union")
+    assert bench.walk_kernel(1, 1048576, 0.5) == ("k_walk_fp64_lanes", "fp64_walk_lanes")

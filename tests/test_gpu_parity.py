@@ -354,11 +354,11 @@ def test_step_graph_equals_direct_launches(dwarf_small, precision):
                                  dict(theta=1.0, criterion="SW93", useQuad=True),
                                  dict(theta=0.7, criterion="TreeCode", useQuad=False)],
                          ids=lambda c: "%s-%g-q%d" % (c["criterion"], c["theta"], c["useQuad"]))
-def test_union_and_per_lane_walks_are_bit_equal(dwarf_small, cfg):
-    """The FP64 walk's forms (nbSetWalkFormCUDA): the warp-union walk, the per-lane walk with
-    and without the early load of the next record, and the automatic choice among them all give
-    each body its CPU walk -- the oracle's accelerations bit for bit, and the same interaction
-    counts."""
+def test_team_and_per_lane_walks_are_bit_equal(dwarf_small, cfg):
+    """The FP64 walk's forms (nbSetWalkFormCUDA) at a size where form 0 is the team walk: it, the
+    per-lane walk with and without the early load of the next record, and the automatic choice
+    (here the team walk at once) all give each body its CPU walk -- the oracle's accelerations bit
+    for bit, and the same interaction counts."""
     from oracle import bindings as ob
     pos, vel, mass, _ = dwarf_small
     ctx = make_ctx(len(mass), **cfg)
@@ -374,15 +374,36 @@ def test_union_and_per_lane_walks_are_bit_equal(dwarf_small, cfg):
             assert tuple(stats[:3]) == tuple(cnt), form
             steps[form] = stats[3]
             assert st.walk_form() == form
-    # the per-lane walks run fewer warp iterations than the union walk
+    # a warp of the per-lane walks serves 32 bodies, one of the team walk four
     assert steps[1] == steps[2] < steps[0]
-    # automatic: the first six evaluations cycle twice through the forms, then one is kept
     with _gpu_state(ctx, pos, vel, mass) as st:
         assert st.walk_form() == -1
-        for _ in range(7):
+        for _ in range(2):
             assert st.gravMap(ctx) == 0
             assert bits_equal(st.accels(), acc)
-        assert st.walk_form() in (0, 1, 2)
+            assert st.walk_form() == 0
+
+
+@pytest.mark.parametrize("quad", [True, False])
+def test_union_walk_counts(quad):
+    """Form 0 above the team walk's lines: the warp's union of paths, the same counts as the oracle's
+    and one warp iteration for every node that any lane visits."""
+    from oracle import bindings as ob
+    from milkywayathome_client_b200 import models
+    n = 12545                                   # the last warp has one body
+    pos, vel, mass, _ = models.plummer_plummer_dwarf(n, seed=2)
+    ctx = make_ctx(n, theta=0.19, useQuad=quad)
+    rc, acc, _, _, cnt = ob.grav_map(ctx.struct, pos, mass, ctx.treeRSize, counts=True)
+    steps = {}
+    for form in (0, 1):
+        with _gpu_state(ctx, pos, vel, mass) as st:
+            st.set_walk_form(form)
+            st.set_counting(True)
+            assert st.gravMap(ctx) == rc == 0
+            stats = st.walk_stats()
+            assert bits_equal(st.accels(), acc) and tuple(stats[:3]) == tuple(cnt)
+            steps[form] = stats[3]
+    assert steps[0] > steps[1]
 
 
 @pytest.mark.parametrize("form", [0, 1, 2])
