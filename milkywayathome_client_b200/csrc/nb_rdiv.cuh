@@ -74,6 +74,16 @@ NB_RD bool nb_pos_exp_in(double x)
     return nb_hi32(x) - ((unsigned) (LO + 1023) << 20) < (unsigned) (HI - LO) << 20;
 }
 
+// +0 or -0
+NB_RD bool nb_is_zero(double x)
+{
+#if defined(__CUDA_ARCH__)
+    return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0;
+#else
+    return x == 0.0;
+#endif
+}
+
 // The first 20 bits of the fraction are ones: holds the divisors above 2 - 2^-21 (scaled), for which
 // the bounds do not stand, and their squares
 NB_RD bool nb_near_ones(double x) { return (nb_hi32(x) & 0xfffffu) == 0xfffffu; }

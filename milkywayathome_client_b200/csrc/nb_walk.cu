@@ -52,7 +52,8 @@ __global__ void k_pack_walk(const double4* __restrict__ nodePM, const double* __
 // and 2^700 keep every intermediate and every residual normal; the operators take the rest, and
 // the divisors next to an all-ones significand.
 // ALWAYS: the quadrupole's factors are formed whether or not this lane's node is a cell (no branch).
-// Returns whether the operands are in those ranges.
+// Returns whether the operands are in those ranges (a mass of +-0, for which mor3 comes out as a
+// zero all the same, is not: only the direct sum meets one, and asks nb_mor3_shared again).
 template <bool ALWAYS>
 __device__ __forceinline__ bool nb_radial_shared(double s, double m, bool cell, double drQdr,
                                                  double& mor3, double& dr5inv, double& phiQ)
@@ -70,6 +71,12 @@ __device__ __forceinline__ bool nb_radial_shared(double s, double m, bool cell, 
         ok = ok && (!cell || (nb_exp_in<-700, 700>(a) && !nb_near_ones(t)));
     }
     return ok;
+}
+
+// Whether nb_radial_shared's mor3 stands.
+__device__ __forceinline__ bool nb_mor3_shared(double s, double m)
+{
+    return nb_pos_exp_in<-100, 100>(s) && !nb_near_ones(s) && (nb_exp_in<-700, 700>(m) || nb_is_zero(m));
 }
 
 // The operators' forms.
@@ -531,7 +538,8 @@ void nb_launch_body_epilogue(const double* px, const double* py, const double* p
 // chains (116 cycles a source where the pipe takes 62).  A thread a body in blocks of 256, one
 // chain at a time, took 2.24 ms at 10,007 bodies and 0.23 at 1,000; now 0.59 and 0.041.  H = 1 / 2 /
 // 4 in ms: 4,000 bodies 0.244 / 0.175 / 0.135, 7,000 0.420 / 0.304 / 0.357, 10,007 0.593 / 0.693 /
-// 0.779, 20,000 2.03 / 2.11 / 2.50 (4.46 before), 30,000 3.03 / 4.08 / 5.20.
+// 0.779, 20,000 2.03 / 2.11 / 2.50 (4.46 before), 30,000 3.03 / 4.08 / 5.20.  With every eighth body a
+// test particle 20,000 take 2.46 (6.40 with the operators for every group that holds one).
 constexpr int EXACT_TILE = 256;
 constexpr int EXACT_UNROLL = 8;
 template <int H>
@@ -588,10 +596,15 @@ k_direct_fp64(const double* __restrict__ px, const double* __restrict__ py,
 #pragma unroll
         for (int u = 0; u < U; ++u)
             ok &= nb_radial_shared<false>(r2[u], mm[u], false, 0.0, mor3[u], dr5inv, phiQ);
-        if (!ok)
+        if (!ok) {                                      // test particles among the sources, or worse
+            ok = true;
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-                nb_radial_general(r2[u], mm[u], false, 0.0, mor3[u], dr5inv, phiQ);
+            for (int u = 0; u < U; ++u) ok &= nb_mor3_shared(r2[u], mm[u]);
+            if (!ok)
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    nb_radial_general(r2[u], mm[u], false, 0.0, mor3[u], dr5inv, phiQ);
+        }
         // the sum never is -0, so a zero term leaves it as it is
 #pragma unroll
         for (int u = 0; u < U; ++u)

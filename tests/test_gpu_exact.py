@@ -35,6 +35,24 @@ def test_operands_outside_the_shared_ranges(eps2, scale):
         assert np.array_equal(st.accels(), want, equal_nan=True)
 
 
+@pytest.mark.parametrize("every", [1, 3, 8])
+def test_test_particles(every):
+    """Massless sources of either sign of zero beside massive ones, a subnormal mass among them."""
+    from milkywayathome_client_b200 import NBodyState, models
+    from oracle import bindings as ob
+    n = 1003
+    pos, vel, mass, _ = models.plummer_plummer_dwarf(n, seed=4)
+    mass = mass.copy()
+    mass[::every] = 0.0
+    mass[::2 * every] = -0.0
+    mass[500:502] = 5e-324, -3e-310
+    ctx = make_ctx(n, criterion="Exact")
+    rc, want, _, _ = ob.grav_map(ctx.struct, pos, mass, ctx.treeRSize)
+    with NBodyState.create(ctx, pos, vel, mass, gravmap=False) as st:
+        assert st.gravMap(ctx) == rc
+        assert bits_equal(st.accels(), want)
+
+
 @pytest.mark.parametrize("criterion,form", [("Exact", 0), ("TreeCode", 0), ("TreeCode", 1)])
 def test_operands_next_to_midpoints(criterion, form):
     """Two bodies so close that s = |dr|^2 + eps^2 is eps^2: the softened distances whose root or

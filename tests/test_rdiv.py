@@ -62,7 +62,7 @@ extern "C" void ranges(const double* x, int n, int* out)
 {
     for (int i = 0; i < n; ++i)
         out[i] = nb_exp_in<-700, 700>(x[i]) | nb_pos_exp_in<-100, 100>(x[i]) << 1 |
-                 nb_near_ones(x[i]) << 2;
+                 nb_near_ones(x[i]) << 2 | nb_is_zero(x[i]) << 3;
 }
 '''
 
@@ -265,9 +265,9 @@ def test_ranges(lib):
     with np.errstate(invalid="ignore"):
         want = ((ax >= 2.0 ** -700) & (ax < 2.0 ** 700)).astype(int) | \
                (((x >= 2.0 ** -100) & (x < 2.0 ** 100)).astype(int) << 1)
-    assert (out & 3).tolist() == want.tolist()
+    assert (out & 3).tolist() == want.tolist() and (out >> 3 & 1).tolist() == (x == 0.0).tolist()
     x = np.array([2.0 - 2.0 ** -52, 2.0 - 2.0 ** -20, 2.0 - 2.0 ** -19, 1.0, 4.0 - 2.0 ** -51])
     out = np.empty(len(x), np.int32)
     lib.ranges(x.ctypes.data_as(ctypes.c_void_p), ctypes.c_int(len(x)),
                out.ctypes.data_as(ctypes.c_void_p))
-    assert (out >> 2).tolist() == [1, 1, 0, 0, 1]
+    assert (out >> 2 & 1).tolist() == [1, 1, 0, 0, 1]
