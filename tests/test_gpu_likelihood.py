@@ -174,6 +174,68 @@ def test_batch_likelihood_matches_single_states():
         assert np.array_equal(out[k], lk, equal_nan=True)
 
 
+def _beta_dispersions(params, pos, types):
+    """The beta dispersions and their errors of every bin, restated from nbRemoveOutliers and
+    nbCalcDisp (nbody/src/nbody_mass.c:190-316): sums in body order, IterMax outlier passes, each
+    against the mean and dispersion of the pass before."""
+    import torch
+    from milkywayathome_client_b200.adjoint import lambda_beta
+    lam, beta = (t.numpy() for t in lambda_beta(torch.from_numpy(pos), params.phi, params.theta,
+                                                params.psi, params.sunGCDist))
+    li = np.floor((lam - params.lambdaStart) / ((params.lambdaEnd - params.lambdaStart) / params.lambdaBins))
+    bi = np.floor((beta - params.betaStart) / ((params.betaEnd - params.betaStart) / params.betaBins))
+    inside = (types >= 0) & (li >= 0) & (li < params.lambdaBins) & (bi >= 0) & (bi < params.betaBins)
+    bins = np.where(inside, li * params.betaBins + bi, -1).astype(int)
+    out = np.zeros((2, params.nbins))
+    for b in range(params.nbins):
+        v = beta[bins == b]
+        keep, var, err = np.ones(len(v), bool), 0.0, 0.0
+        for k in range(params.IterMax + 1):
+            if k > 0:
+                n = keep.sum()
+                mean = v[keep].sum() / n if n else np.nan
+                keep = np.abs(mean - v) < params.BetaSigma * var
+            n = int(keep.sum())
+            if n > 10:
+                s, q = v[keep].sum(), (v[keep] ** 2).sum()
+                d = q / (n - 1) - (n / (n - 1)) * (s / n) ** 2
+                var = np.sqrt(d * (params.BetaCorrect if k else 1.0))
+                err = np.sqrt((n + 1) / (n * (n - 1))) * var
+        out[:, b] = var, err
+    return out
+
+
+@pytest.mark.parametrize("iter_max", [0, 1, 6])
+def test_dispersions_of_many_bins(iter_max):
+    """Batches with more bins than there are warps to take one each: empty bins, bins of up to ten
+    bodies, of one and of several fetches.  Against a plain restatement, whose sums in another
+    order differ by about 1e-13 of the squared values, a thousand times the dispersion's square at
+    most; and bit for bit what each dwarf gives alone."""
+    from milkywayathome_client_b200 import HistogramParams, NBodyBatch, NBodyState
+    params = HistogramParams(lambdaStart=-180.0, lambdaEnd=180.0, lambdaBins=50, betaStart=-90.0,
+                             betaEnd=90.0, betaBins=8, IterMax=iter_max)
+    rng = np.random.default_rng(7)
+    sizes = [40, 300, 3000, 9000] * 15
+    pos = [20.0 * rng.standard_normal((n, 3)) for n in sizes]
+    pos[3][:, 2] *= 0.05                         # full bins along the plane
+    types = [np.where(rng.uniform(size=n) < 0.9, 1, -1) for n in sizes]
+    vel = [np.zeros((n, 3)) for n in sizes]
+    with NBodyBatch([(n, 1e-3, 1e-3, 4.0) for n in sizes]) as bt:
+        bt.set_bodies(np.concatenate(pos), np.concatenate(vel), np.ones(sum(sizes)))
+        bt.set_types(np.concatenate(types))
+        counts, _, _, comps = bt.histogram(params, components=True)
+    assert counts.size > 148 * 32 * 4 and counts.max() > 64 and (counts == 0).any()
+    for d in (0, 1, 2, 3, 59):
+        np.testing.assert_allclose(comps[d, 0], _beta_dispersions(params, pos[d], types[d]),
+                                   rtol=1e-9, atol=0.0)
+        st = NBodyState(sizes[d], 0)
+        with st:
+            st.set_bodies(pos[d], vel[d], np.ones(sizes[d]), 4.0)
+            st.set_types(types[d])
+            one = st.histogram(params, components=True)
+        assert np.array_equal(one[0][0], counts[d]) and np.array_equal(one[3][0], comps[d])
+
+
 # ---- two-dimensional histograms (betaBins > 1): the EMD by the transportation simplex ----
 def _orphan_params_2d(beta_bins, **flags):
     from milkywayathome_client_b200 import HistogramParams
