@@ -277,7 +277,7 @@ static NBodyCudaStatus nb_alloc_bodies(NBodyCudaState* st, int n)
     NB_CHECK(nb_alloc(&b.sort.idxA, N)); NB_CHECK(nb_alloc(&b.sort.idxB, N));
     const int tiles = (int) ((N + 2047) / 2048);
     NB_CHECK(nb_alloc(&b.sort.hist, 256 * (size_t) tiles));
-    NB_CHECK(nb_alloc(&b.sort.histTmp, (size_t) std::max(256, nb_scan_tmp_ints(256 * tiles))));
+    NB_CHECK(nb_alloc(&b.sort.totals, (size_t) 256));
     b.sort.capTiles = tiles;
     NB_CHECK(nb_alloc(&b.gx, N)); NB_CHECK(nb_alloc(&b.gy, N)); NB_CHECK(nb_alloc(&b.gz, N));
     NB_CHECK(nb_alloc(&b.delta, N)); NB_CHECK(nb_alloc(&b.cum, N));
@@ -294,7 +294,7 @@ static void nb_free_all(NBodyCudaState* st)
     double* d[] = {b.px, b.py, b.pz, b.vx, b.vy, b.vz, b.ax, b.ay, b.az, b.mass, st->stage};
     for (double* p : d) cudaFree(p);
     cudaFree(b.sort.keyA); cudaFree(b.sort.keyB); cudaFree(b.sort.idxA); cudaFree(b.sort.idxB);
-    cudaFree(b.sort.hist); cudaFree(b.sort.histTmp);
+    cudaFree(b.sort.hist); cudaFree(b.sort.totals);
     cudaFree(b.gx); cudaFree(b.gy); cudaFree(b.gz);
     cudaFree(b.delta); cudaFree(b.cum); cudaFree(b.scanTmp); cudaFree(b.bodyNode);
     cudaFree(b.sc);

@@ -267,7 +267,7 @@ struct NbSortBuffers {
     unsigned long long* keyA; unsigned long long* keyB;
     unsigned int* idxA; unsigned int* idxB;
     unsigned int* hist;    // 256 * nTiles
-    int* histTmp;          // tile sums of the scan over hist
+    unsigned int* totals;  // of every digit, 256
     int capTiles;
 };
 // Sorts (keyA, idxA) by key in place (result in keyA/idxA); n items.

@@ -250,7 +250,8 @@ __device__ __forceinline__ double ic_integrand(const Model& m, double ri, double
 // each: with a thread a body the warps waited for their longest body and a few long ones set
 // the time (eight dwarfs of 4,096 to 65,536 bodies: 185 -> 83 ms, and 62 with the shared
 // reciprocals of NbIcPlummerModel::stencils).  FP64 issue and its dependences bound it now; five
-// resident blocks (96 registers, a few spilled) beat four by 2 % and three by 10 %.
+// resident blocks (96 registers; 300 bytes of spill stores with two Plummer components, 644 with
+// others) beat four by 2 % and three by 10 %.
 struct NbIcWarp {
     int lane;
     double* terms;              // 32 doubles of shared memory

@@ -78,7 +78,7 @@ __global__ void k_pack_f32(const double4* __restrict__ nodePM, const double* __r
 // Walk: warp-parallel depth-first traversal.  Each step pops up to 32 nodes from the warp's
 // stack (one per lane), tests them at once, appends visited bodies and accepted cells to two
 // per-warp interaction lists in shared memory and pushes the children of opened cells
-// (explicit child lists built by k_pack_f32).  Popping from the top keeps the stack sorted by
+// (the child lists of the tree's link phase).  Popping from the top keeps the stack sorted by
 // depth, so at most 8 x 32 nodes of any one depth are ever on it: 256 x 63 levels bounds it
 // (NB_GROUP_STACK).  A full list is evaluated by all 32 lanes at once (each lane for its own
 // body, entries read as shared-memory broadcasts), FP32 with FMA and nb_rsqrt; partial sums go

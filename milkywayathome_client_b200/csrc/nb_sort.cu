@@ -250,7 +250,6 @@ static void rs_passes(NbSortBuffers& b, int n, const int* group, cudaStream_t s)
     unsigned long long* kin = b.keyA; unsigned long long* kout = b.keyB;
     unsigned int* iin = b.idxA; unsigned int* iout = b.idxB;
     const int passes = group ? 10 : 8;
-    unsigned int* totals = (unsigned int*) b.histTmp;
     const int rowThreads = nTiles > 512 ? 1024 : nTiles > 128 ? 512 : 128;
     for (int pass = 0; pass < passes; ++pass) {
         const bool grouped = pass >= 8;
@@ -259,13 +258,13 @@ static void rs_passes(NbSortBuffers& b, int n, const int* group, cudaStream_t s)
             k_rs_hist<true><<<nTiles, RS_THREADS, 0, s>>>(kin, iin, group, n, shift, b.hist, nTiles);
         else
             k_rs_hist<false><<<nTiles, RS_THREADS, 0, s>>>(kin, iin, nullptr, n, shift, b.hist, nTiles);
-        k_rs_rows<<<256, rowThreads, 0, s>>>(b.hist, nTiles, totals);
+        k_rs_rows<<<256, rowThreads, 0, s>>>(b.hist, nTiles, b.totals);
         if (grouped)
             k_rs_scatter<true><<<nTiles, RS_THREADS, 0, s>>>(kin, iin, kout, iout, group, n, shift,
-                                                             b.hist, totals, nTiles);
+                                                             b.hist, b.totals, nTiles);
         else
             k_rs_scatter<false><<<nTiles, RS_THREADS, 0, s>>>(kin, iin, kout, iout, nullptr, n,
-                                                              shift, b.hist, totals, nTiles);
+                                                              shift, b.hist, b.totals, nTiles);
         nb_count_launch(3);
         unsigned long long* tk = kin; kin = kout; kout = tk;
         unsigned int* ti = iin; iin = iout; iout = ti;

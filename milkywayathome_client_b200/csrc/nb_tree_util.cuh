@@ -147,9 +147,8 @@ __device__ __forceinline__ double4 nb_ld_pm(const double4* p)
     return make_double4(a.x, a.y, b.x, b.y);
 }
 
-
-// A cell's children in octant order, from its slot's two int4 (-1 past the last).  L2 loads, as
-// the other phases of the same kernel may have written them.
+// A cell's children in octant order, from its slot's two int4 (-1 past the last).  L2 loads: a list is
+// read once, and the records it leads to are L2 loads anyway.
 __device__ __forceinline__ void nb_load_kids(const int4* kids, int slot, int (&k)[8])
 {
     const int4 a = __ldcg(kids + 2 * (size_t) slot), b = __ldcg(kids + 2 * (size_t) slot + 1);

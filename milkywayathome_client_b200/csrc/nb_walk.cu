@@ -743,11 +743,6 @@ __global__ void k_ext_only(const double* __restrict__ pos, double* __restrict__ 
 
 // ---- host launchers ----
 
-void nb_launch_body_epilogue(const double* px, const double* py, const double* pz, double* ax,
-                             double* ay, double* az, double* vx, double* vy, double* vz,
-                             const NbWalkParams& wp, const NbPot& pot, const NbScalars* sc,
-                             int numSMs, cudaStream_t s, const NbForest* forest);
-
 void nb_launch_pack_walk(const NbTreeBuffers& b, int capNodes, bool slots, cudaStream_t s)
 {
     k_pack_walk<<<min((capNodes + 255) / 256, 4096), 256, 0, s>>>(
@@ -816,25 +811,19 @@ void nb_launch_walk_fp64(const NbTreeBuffers& b, int capNodes, const NbWalkParam
 #define NB_LANES_ARGS b.walkRec, b.sort.idxA, b.px, b.py, b.pz, b.ax, b.ay, b.az, wp, b.sc, f
 #define NB_TEAM_ARGS                                                                          \
     b.walkRec, (const int*) b.walkKids, b.sort.idxA, b.px, b.py, b.pz, b.ax, b.ay, b.az, wp, b.sc, f
-#define NB_TEAM(FOREST)                                                                       \
+#define NB_TEAM(COUNT, FOREST) k_walk_fp64_team<COUNT, FOREST><<<teamBlocks, WALK_THREADS, 0, s>>>(NB_TEAM_ARGS)
+#define NB_LANES(COUNT, FOREST, PATH)                                                         \
+    k_walk_fp64_lanes<COUNT, FOREST, PATH><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS)
+#define NB_WALK(COUNT, FOREST)                                                                \
     do {                                                                                      \
-        if (count) k_walk_fp64_team<true, FOREST><<<teamBlocks, WALK_THREADS, 0, s>>>(NB_TEAM_ARGS); \
-        else k_walk_fp64_team<false, FOREST><<<teamBlocks, WALK_THREADS, 0, s>>>(NB_TEAM_ARGS);    \
+        if (kernel == NB_WALK_TEAM) NB_TEAM(COUNT, FOREST);                                   \
+        else if (kernel == NB_WALK_EARLY) NB_LANES(COUNT, FOREST, LANES_EARLY);               \
+        else if (kernel == NB_WALK_UNION) NB_LANES(COUNT, FOREST, LANES_UNION);               \
+        else NB_LANES(COUNT, FOREST, LANES_OWN);                                              \
     } while (0)
-#define NB_LANES(FOREST, PATH)                                                                \
-    do {                                                                                      \
-        if (count) k_walk_fp64_lanes<true, FOREST, PATH><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS); \
-        else k_walk_fp64_lanes<false, FOREST, PATH><<<blocks, WALK_THREADS, 0, s>>>(NB_LANES_ARGS);    \
-    } while (0)
-#define NB_WALK(FOREST)                                                                       \
-    do {                                                                                      \
-        if (kernel == NB_WALK_TEAM) NB_TEAM(FOREST);                                          \
-        else if (kernel == NB_WALK_EARLY) NB_LANES(FOREST, LANES_EARLY);                      \
-        else if (kernel == NB_WALK_UNION) NB_LANES(FOREST, LANES_UNION);                      \
-        else NB_LANES(FOREST, LANES_OWN);                                                     \
-    } while (0)
-    if (forest) NB_WALK(true);
-    else NB_WALK(false);
+    if (forest) NB_WALK(false, true);               // a batch does not count
+    else if (count) NB_WALK(true, false);
+    else NB_WALK(false, false);
 #undef NB_WALK
 #undef NB_LANES
 #undef NB_TEAM
