@@ -15,7 +15,7 @@
 // list offsets (k_bin_offsets), and the chunk warps place their bodies (k_bin_scatter, lanes
 // of one bin ranked in lane order).  Finally one warp per (quantity, dwarf, bin) walks its
 // bin's list once per pass -- the initial sums and IterMax outlier passes, each followed by
-// nbCalcDisp -- adding in body order, as the reference does (k_disp_bins): the dispersions
+// nbCalcDisp -- adding in body order, as the reference does (nb_disp_bin): the dispersions
 // and averages equal the reference's bit for bit.  Counts are integers and exact.
 #include "nb_common.cuh"
 #include "nb_crmath.cuh"
@@ -300,11 +300,21 @@ __device__ __forceinline__ void nb_disp_bin(const NbHistPlan& p, int t, int lane
     p.err[t] = err;
 }
 
-// Every warp takes the bins w, w + W, w + 2 W .. of W warps, 32 at a time: of those with up to ten
+// One bin a warp, while they are no more than a few waves of warps.
+__global__ void __launch_bounds__(HW * 32) k_disp_bin(NbHistPlan p)
+{
+    __shared__ double part[HW][2][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int t = blockIdx.x * HW + w;
+    if (t < p.h.nq * p.D * p.B) nb_disp_bin(p, t, lane, part[w]);     // the warp alike
+}
+
+// More bins: every warp takes the bins w, w + W, w + 2 W .. of W warps, 32 at a time: of those with up to ten
 // bodies nothing is left after the first outlier pass (their dispersion, and so its limit, is zero), and
 // their lane writes that down; the others are the warp's, one after another.  Batches of small dwarfs
 // have few others: 500 dwarfs of 200 bodies with 340 bins and seven quantities took 2.59 ms a likelihood
-// with a warp for every bin and 1.87 with a thread.
+// with a warp for every bin, 1.87 with a thread, and take 1.78.  The loop's registers (62 against 52)
+// make this form the slower one for a bin: one dwarf of 10,000 bodies 0.51 ms a likelihood, 0.49 above.
 __global__ void __launch_bounds__(HW * 32) k_disp_bins(NbHistPlan p)
 {
     __shared__ double part[HW][2][32];
@@ -828,7 +838,8 @@ int nb_launch_hist_plan(const NbHistPlan& p, const double* px, const double* py,
         k_bin_offsets<<<1, 1024, 0, s>>>(p);
         k_bin_scatter<<<chunkBlocks, HW * 32, 0, s>>>(p);
         const size_t warpBlocks = std::min((Q + HW - 1) / HW, (size_t) numSMs * 32);
-        k_disp_bins<<<(int) warpBlocks, HW * 32, 0, s>>>(p);
+        if (warpBlocks * HW >= Q) k_disp_bin<<<(int) warpBlocks, HW * 32, 0, s>>>(p);
+        else k_disp_bins<<<(int) warpBlocks, HW * 32, 0, s>>>(p);
         launches += 4;
     }
     nb_count_launch(launches);
