@@ -889,7 +889,8 @@ def run_profile(args):
     pos, vel, mass, _ = bench_input(args.n, SEED_1M)
     ctx, _ = bench_ctx(args.n, args.theta, precision=args.profile)
     with NBodyState(args.n, 0) as st:
-        st.set_walk_form(WALK_FORM if WALK_FORM >= 0 else 0)
+        # unset: the form that the automatic choice keeps at the benchmark's angles
+        st.set_walk_form(WALK_FORM if WALK_FORM >= 0 else 0 if args.n <= 24576 else 1)
         st.set_bodies(pos, vel, mass, ctx.treeRSize)
         st.check("nbGravMap", st.gravMap(ctx))
         st.check("nbGravMap", st.gravMap(ctx))

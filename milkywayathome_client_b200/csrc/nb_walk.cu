@@ -339,15 +339,16 @@ k_walk_fp64_team(const double4* __restrict__ rec, const int* __restrict__ kids,
 // meets exactly its CPU walk's nodes in the CPU's order and sums the same terms in the same
 // order.  Bodies consecutive in path order have walks of similar length, so the warp runs about
 // as many iterations as its longest walk (0.96 of the lane slots do work on the 131k-body dwarf
-// at theta 0.5).  Bound by the L1 data pipe (87 % busy: a 32-byte load is at least eight
-// wavefronts a warp, more with distinct records) and the FP64 pipe (63 %).  Sharing one
+// at theta 0.5).  Bound by the L1 data pipe (88 % busy: a 32-byte load is at least eight
+// wavefronts a warp, more with distinct records) and the FP64 pipe (59 %).  Sharing one
 // reciprocal among the root and the divisions (nb_radial) took the 1,048,576-body dwarf from 28.9
 // to 28.1 ms at theta 0.5 and from 7.05 to 6.54 ms at theta 1.
 // LANES_EARLY: the next node's record is loaded as soon as the opening test has chosen it, before
 // this node's terms are computed, so its latency overlaps the FP64 arithmetic (79 registers
 // against 63: it pays where few warps are resident, up to some 80,000 bodies).
 // LANES_UNION: the warp takes the smallest of its lanes' next nodes, the lanes that are at it do it:
-// one broadcast load a node, but an iteration for every node that any lane visits.  The smaller the
+// one broadcast load a node, but an iteration for every node that any lane visits (FP64 pipe 68 %
+// busy, L1 data pipe 37 %).  The smaller the
 // opening angle, the more of a walk its neighbours share: walks of 1,048,576 bodies, own -> union:
 // theta 0.7 12.4 -> 13.6 ms, 0.5 28.1 -> 28.2, 0.4 49.4 -> 44.2, 0.3 107 -> 84.5, 0.2 302 -> 210; 50,000
 // bodies, early -> union: 0.5 1.89 -> 2.70, 0.25 9.64 -> 9.98, 0.2 15.2 -> 13.6, 0.1 34.2 -> 22.3.
