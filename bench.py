@@ -514,7 +514,7 @@ WALK_FORM_NAMES = {0: "shared (team or union)", 1: "per lane", 2: "per lane, nex
 def walk_kernel(form, n, theta):
     """(kernel, entry of the traffic profile) of a walk form at this size: form 0 is the team walk
     for small systems and the union of a warp's paths, in the per-lane kernel, for others."""
-    if form == 0 and (n <= 12288 or (n <= 32768 and theta >= 0.2)):
+    if form == 0 and (n <= 12288 or (n <= 32768 and theta >= min(0.2, (n - 9000) / 85000))):
         return "k_walk_fp64_team", "fp64_walk_team"
     return "k_walk_fp64_lanes", "fp64_walk_union" if form == 0 else "fp64_walk_lanes"
 

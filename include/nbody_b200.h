@@ -354,9 +354,9 @@ NBodyCudaStatus nbSetStepGraphCUDA(NBodyCudaState* st, int enable);
 
 /* The FP64 force walk's form: 0 shares a warp's node visits -- the team walk (a warp walks for four
  * bodies, eight lanes each evaluating the nodes of one body's path) for systems of up to 12,288
- * bodies, and up to 32,768 at theta >= 0.2; else the union walk (a lane a body, the warp visiting
- * the union of its bodies' paths).  1 walks every body's path in its own lane (a lane idles only
- * once its walk is over; per-lane loads); 2 is the per-lane walk that loads the next node's record
+ * bodies, and up to 32,768 at theta >= 0.2 (less for fewer bodies); else the union walk (a lane a
+ * body, the warp visiting the union of its bodies' paths).  1 walks every body's path in its own
+ * lane (a lane idles only once its walk is over; per-lane loads); 2 is the per-lane walk that loads the next node's record
  * as soon as the opening test has chosen it, overlapping that load with the current node's
  * arithmetic (more registers: faster for some tens of thousands of bodies, slower at a million).
  * -1 (the default) takes the team walk up to 24,576 bodies (12,288 without quadrupoles) at theta >=

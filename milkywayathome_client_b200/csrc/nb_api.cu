@@ -702,6 +702,7 @@ extern "C++" {
 // nothing: 18.8 GB/s by the driver, 12 staged.  Below kStageMin the threads cost more than they save.
 // Every other kind of memory (page-locked, managed, a device pointer given by mistake) goes to
 // cudaMemcpyAsync, whose status the caller gets: a host thread must not write to what it cannot reach.
+// The threads' waits spin: events that block them took two arrays of 30 MB from 4.2 to 10.7 ms.
 static const int kStageSlots = 8;
 static const size_t kStageSlot = (size_t) 1 << 20;
 static const size_t kStageMin = (size_t) 4 << 20;

@@ -119,9 +119,11 @@ __device__ __forceinline__ void nb_radial(double s, double m, bool need, bool ce
 // 0.542; without them, when the additions are most of a node's work, 5,000 0.190 -> 0.156, 12,000
 // 0.217 -> 0.211 (0.7: 0.362 -> 0.367, 0.5: 0.684 -> 0.713), 16,384 0.218 -> 0.306, 32,768 0.254 ->
 // 0.529.  Hence the automatic choice's two lines.  Small opening angles take few cells and many
-// bodies, whose work is mostly the additions again: quadrupoles, 24,000 bodies, union -> team: theta
-// 0.2 8.23 -> 7.85, 0.1 12.1 -> 15.7, 0.05 12.1 -> 20.4; 12,000: 0.1 5.94 -> 5.12, 0 7.09 -> 11.8.  So
-// form 0 is the team walk up to the smaller line, and up to TEAM_MAX_BODIES from TEAM_THETA on.
+// bodies, whose work is mostly the additions again.  With quadrupoles, union -> team: 12,000 bodies,
+// theta 0.05 6.09 -> 5.65, 0 7.09 -> 11.8; 14,000, 0.1 7.08 -> 6.39; 16,384, 0.1 8.02 -> 8.72, 0.05 8.35 ->
+// 12.4; 20,000, 0.15 8.79 -> 8.49, 0.1 9.84 -> 11.6; 24,000, 0.2 8.23 -> 7.85, 0.15 10.2 -> 11.3; 32,768, 0.2
+// 11.0 -> 10.2, 0.15 13.5 -> 16.0.  So form 0 is the team walk up to the smaller line, and up to
+// TEAM_MAX_BODIES where theta >= min(TEAM_THETA, (bodies - 9,000) / 85,000).
 constexpr int TEAM_BODIES = 4;
 constexpr int TEAM_MAX_BODIES = 32768;
 constexpr int TEAM_AUTO_QUAD = 24576, TEAM_AUTO_MONO = 12288;
@@ -754,8 +756,9 @@ void nb_launch_pack_walk(const NbTreeBuffers& b, int capNodes, bool slots, cudaS
 // Form 0's kernel, and where it is the team walk and the fastest form without timing.
 int nb_walk_shared(int n, double theta)
 {
-    return n <= TEAM_AUTO_MONO || (n <= TEAM_MAX_BODIES && theta >= TEAM_THETA) ? NB_WALK_TEAM
-                                                                               : NB_WALK_UNION;
+    const double least = fmin(TEAM_THETA, (n - 9000) / 85000.0);
+    return n <= TEAM_AUTO_MONO || (n <= TEAM_MAX_BODIES && theta >= least) ? NB_WALK_TEAM
+                                                                          : NB_WALK_UNION;
 }
 bool nb_walk_team_auto(int n, int useQuad, double theta)
 {

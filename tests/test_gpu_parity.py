@@ -390,9 +390,9 @@ def test_union_walk_counts(quad):
     and one warp iteration for every node that any lane visits."""
     from oracle import bindings as ob
     from milkywayathome_client_b200 import models
-    n = 12545                                   # the last warp has one body
+    n = 16385                                   # the last warp has one body
     pos, vel, mass, _ = models.plummer_plummer_dwarf(n, seed=2)
-    ctx = make_ctx(n, theta=0.19, useQuad=quad)
+    ctx = make_ctx(n, theta=0.08, useQuad=quad)
     rc, acc, _, _, cnt = ob.grav_map(ctx.struct, pos, mass, ctx.treeRSize, counts=True)
     steps = {}
     for form in (0, 1):

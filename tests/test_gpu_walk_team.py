@@ -105,7 +105,7 @@ def test_the_automatic_choice_follows_the_context():
 
 
 @pytest.mark.parametrize("n,theta", [(32767, 0.9), (32768, 0.9), (32769, 0.9), (12288, 0.1),
-                                     (12289, 0.1), (12289, 0.2)])
+                                     (12289, 0.03), (12289, 0.05), (20001, 0.12), (20001, 0.14)])
 def test_both_sides_of_the_line_equal_the_per_lane_walk(n, theta):
     """Form 0: the team walk on one side of its lines, the union of a warp's paths on the other."""
     from milkywayathome_client_b200 import models
