@@ -781,7 +781,7 @@ bool nb_walk_team_auto(int n, int useQuad, double theta)
 //     0.746 -> 0.709; 1 of 40,000, 0.3 5.8 -> 7.1), and less without quadrupoles (own path -> union: 20
 //     of 10,000, 0.5 2.84 -> 2.87, 0.4 4.22 -> 3.77; 100 of 10,000, 0.7 5.70 -> 6.30, 0.5 10.6 -> 10.3).
 //     Not where a walk is nearly all bodies (early load -> union: 50 dwarfs of 1,000, 0.1 0.907 -> 1.18)
-//     nor for the smallest dwarfs (200 of 200: 0.5 0.361 -> 0.430).
+//     nor for the smallest dwarfs (80 of 500: 0.3 0.557 -> 0.594; 200 of 200: 0.5 0.361 -> 0.430).
 //   * Else own paths, with the early load while few warps are resident (own -> early, theta 0.7: 65,536
 //     bodies 1.04 -> 0.97, 80,000 1.11 -> 1.04, 96,758 1.19 -> 1.20, 131,072 1.33 -> 1.57).
 constexpr int EARLY_MAX_BODIES = 81920;
@@ -796,7 +796,7 @@ int nb_walk_batch(int n, int dwarfs, int useQuad, double theta)
     const bool many = n >= UNION_MANY_BODIES;
     const double limit = useQuad ? (many ? 990.0 : 440.0 * (full * full))
                                  : (many ? 1040.0 : full >= 0.75 ? 104.0 * (full * full) : -1.0);
-    if (mean >= 400.0 && cells * full >= 8.0 && shared <= limit && (useQuad || theta <= 0.5))
+    if (mean >= 600.0 && cells * full >= 8.0 && shared <= limit && (useQuad || theta <= 0.5))
         return NB_WALK_UNION;
     return n <= EARLY_MAX_BODIES ? NB_WALK_EARLY : NB_WALK_LANES;
 }
