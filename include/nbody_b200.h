@@ -360,7 +360,7 @@ NBodyCudaStatus nbSetStepGraphCUDA(NBodyCudaState* st, int enable);
  * as soon as the opening test has chosen it, overlapping that load with the current node's
  * arithmetic (more registers: faster for some tens of thousands of bodies, slower at a million).
  * -1 (the default) takes the team walk up to 24,576 bodies (12,288 without quadrupoles) at theta >=
- * 0.2, asked at every evaluation; else it cycles twice through forms 1 and 2 (and 0 at theta < 0.5)
+ * 0.2 (0.04 up to 12,288 with quadrupoles), asked at every evaluation; else it cycles twice through forms 1 and 2 (and 0 at theta < 0.5)
  * over a state's first four (six) uncounted FP64 tree evaluations, with quadrupoles and without and
  * on both sides of theta 0.5 each by its own, times the second round (the first launch of each
  * kernel also loads it) and keeps the fastest.  Every form gives every body exactly its CPU walk

@@ -128,6 +128,9 @@ constexpr int TEAM_BODIES = 4;
 constexpr int TEAM_MAX_BODIES = 32768;
 constexpr int TEAM_AUTO_QUAD = 24576, TEAM_AUTO_MONO = 12288;
 constexpr double TEAM_THETA = 0.2;
+// with quadrupoles and up to the smaller line it is the fastest form down to this angle (10,000 bodies at
+// 0.05: early load 5.64, team 4.43; 12,000: 6.81, 5.65; at 0: 5.53, 11.8)
+constexpr double TEAM_SMALL_THETA = 0.04;
 constexpr int TEAM_LANES = 32 / TEAM_BODIES;                // 8: a cell's children
 constexpr unsigned TEAM_ALL = (1u << TEAM_BODIES) - 1u;     // every body of the warp
 constexpr unsigned TEAM_FIRST = 0x11111111u;                // the lanes with b = 0
@@ -762,6 +765,7 @@ int nb_walk_shared(int n, double theta)
 }
 bool nb_walk_team_auto(int n, int useQuad, double theta)
 {
+    if (useQuad && n <= TEAM_AUTO_MONO) return theta >= TEAM_SMALL_THETA;
     return n <= (useQuad ? TEAM_AUTO_QUAD : TEAM_AUTO_MONO) && theta >= TEAM_THETA;
 }
 

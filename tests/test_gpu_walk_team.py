@@ -63,6 +63,18 @@ def test_the_timed_choice(n, quad, theta, evaluations):
         assert st.walk_form() in ((0, 1, 2) if evaluations == 6 else (1, 2))
 
 
+@pytest.mark.parametrize("n,quad,theta", [(1500, True, 0.04), (12288, True, 0.05), (12289, True, 0.2),
+                                          (24576, True, 0.2), (12288, False, 0.2)])
+def test_the_team_walk_by_rule(n, quad, theta):
+    from milkywayathome_client_b200 import NBodyState, models
+    pos, vel, mass, _ = models.plummer_plummer_dwarf(n, seed=6)
+    ctx = make_ctx(n, theta=theta, useQuad=quad)
+    _, want = _acc(ctx, pos, vel, mass, 1)
+    with NBodyState.create(ctx, pos, vel, mass, gravmap=False) as st:
+        assert st.gravMap(ctx) == 0 and st.walk_form() == 0
+        assert bits_equal(st.accels(), want)
+
+
 @pytest.mark.parametrize("sizes,theta,quad", [
     ((3100, 2900, 3200, 3088), 0.5, True), ((3100, 2900, 3200, 3088), 0.0, True),   # 12,288 in all
     ((3100, 2900, 3201, 3088), 0.5, True), ((3100, 2900, 3201, 3088), 0.25, True),
